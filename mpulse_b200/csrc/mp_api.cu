@@ -73,6 +73,7 @@ namespace {
 constexpr int kFaceOrderAll[6] = {FACE_NORTH, FACE_SOUTH, FACE_EAST, FACE_WEST, FACE_UP, FACE_DOWN};
 const int kFaceOrderZ[2] = {FACE_UP, FACE_DOWN};
 thread_local char g_create_err[512];
+constexpr size_t kKerrBytes = size_t(kKerrSlots) * kKerrStride * sizeof(unsigned long long);
 
 constexpr int face_dim(int f) {
   return (f == FACE_EAST || f == FACE_WEST) ? 0 : (f == FACE_NORTH || f == FACE_SOUTH) ? 1 : 2;
@@ -772,8 +773,8 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
   }
   MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_status), ST_COUNT * sizeof(int)), "status allocation");
   MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_status), ST_COUNT * sizeof(int)), "pinned allocation");
-  MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_kerr), 2 * sizeof(unsigned long long)), "counter allocation");
-  MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_kerr), 2 * sizeof(unsigned long long)), "pinned allocation");
+  MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_kerr), kKerrBytes), "counter allocation");
+  MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_kerr), kKerrBytes), "pinned allocation");
   MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_diag), size_t(g.nz + 3) * sizeof(double)), "diagnostics allocation");
   MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_diag), 2 * sizeof(double)), "pinned allocation");
 
@@ -1495,13 +1496,16 @@ int mp_kernel_times(mp_ctx *c, int n_steps, double *e_ms, double *b_ms, double *
 int mp_kerr_counts(mp_ctx *c, long long *solves, long long *iterations) {
   if (!c || !solves || !iterations) return MP_ERR_INVALID;
   cudaSetDevice(c->cfg.device);
-  cudaError_t e = cudaMemcpyAsync(c->h_kerr, c->d_kerr, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+  cudaError_t e = cudaMemcpyAsync(c->h_kerr, c->d_kerr, kKerrBytes, cudaMemcpyDeviceToHost,
                                   c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_kerr, 0, 2 * sizeof(unsigned long long), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_kerr, 0, kKerrBytes, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "Kerr counter read");
-  *solves = (long long)c->h_kerr[0];
-  *iterations = (long long)c->h_kerr[1];
+  *solves = *iterations = 0;
+  for (int q = 0; q < kKerrSlots; ++q) {
+    *solves += (long long)c->h_kerr[q * kKerrStride];
+    *iterations += (long long)c->h_kerr[q * kKerrStride + 1];
+  }
   return MP_OK;
 }
 

@@ -135,7 +135,12 @@ __device__ __forceinline__ double nl_newton(double E, double eps, double chi, do
 
 // Per-thread counts of the Kerr solves a thread ran ([0]: cells in which the
 // Newton solve ran, [1]: the iterations they took), added to the context's
-// counters once per warp when the thread's z-march ends.
+// counters once per warp when the thread's z-march ends.  The counters are
+// kKerrSlots pairs, each in a cache line of its own, and warps of different
+// blocks take different ones: with a single pair every warp's two atomics went
+// to one address, one after the other, and took longer than the march itself
+// where it is short (ten steps of fdtd-nl, 101 x 75 x 163, FP64: 0.786 ms with
+// one pair, 0.608 ms with kKerrSlots; no change where a march is 20 planes).
 struct KerrCount {
   unsigned solves = 0, iters = 0;
 };
@@ -148,6 +153,8 @@ __device__ __forceinline__ void flush_kerr_count(unsigned long long *dst, const 
   const unsigned b = __reduce_add_sync(m, kc.iters);
   const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
   if (lane == __ffs(m) - 1 && a != 0u) {
+    const unsigned block = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    dst += (block % kKerrSlots) * kKerrStride;
     atomicAdd(dst, (unsigned long long)a);
     atomicAdd(dst + 1, (unsigned long long)b);
   }

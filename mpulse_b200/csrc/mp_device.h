@@ -28,6 +28,9 @@ enum Face { FACE_NORTH = 0, FACE_SOUTH, FACE_WEST, FACE_EAST, FACE_UP, FACE_DOWN
 // their array and skipped.
 enum StatusSlot { ST_NEWTON = 0, ST_NONFINITE = 1, ST_TIMEOUT = 2, ST_BOUNDS = 3, ST_COUNT = 4 };
 
+// Slots of the Kerr counters and the words from one to the next (128 bytes).
+static const int kKerrSlots = 256, kKerrStride = 16;
+
 // Tile of the TMA-staged kernels (mp_step_tma.cu): 32 x 8 columns.
 static const int kTmaTileX = 32, kTmaTileY = 8;
 
@@ -122,7 +125,9 @@ struct EParams {
   int src_mult;           // how many injectors share the plane (each adds it once)
   SourcePlane<T> src[4];
   int *status;
-  unsigned long long *kerr_count;  // [0] Kerr solves, [1] their Newton iterations (accumulated)
+  // kKerrSlots counters kKerrStride words apart: [0] Kerr solves, [1] their
+  // Newton iterations (accumulated; the sum over the slots counts)
+  unsigned long long *kerr_count;
   long long n_field;      // elements of each field and history array
   long long n_psi;        // pairs of each PLRC accumulator array
 
