@@ -313,91 +313,28 @@ __device__ __forceinline__ void cell_coef(const EParams<T> &p, int i, int j, int
   }
 }
 
-// SPECIAL = false: the caller guarantees that no CPML face contains the cell
-// and that k is no injection plane; the face and source code is left out.
-// PLASMA: *pc holds the plasma plug-ins' values of the cell (plasma_cell).
-template <typename T, int MODE, int NP, bool DESIGN = false, bool SPECIAL = true, bool PLASMA = false>
-__device__ __forceinline__ void e_cell(const EParams<T> &p, int i, int j, int k, long long col, bool med,
-                                       unsigned cmask, const EIn<T> &v, T ikx, T iky, T ikz,
-                                       typename Vec2<T>::type (&q)[NP > 0 ? NP : 1][3], T &exn, T &eyn,
-                                       T &ezn, KerrCount &kc, const PlasmaCell<T> *pc = nullptr) {
+// The medium coefficients with the conductivity: numer - sig and denom + sig
+// (fdtd_plrc.cpp:188-196, :356-359).
+template <typename T, int NP>
+__device__ __forceinline__ void plasma_coef(const EParams<T> &p, T sig, CellCoef<T, NP> &lc) {
+  lc.numer = lc.numer - sig;
+  lc.inv_denom = T(1) / (p.denom_t + sig);
+  lc.inv_denom_lo = T(0);
+  lc.chi_over_denom = p.chi_raw / (p.denom_d + (double)sig);
+}
+
+// The E update of one cell from its old E, the curl of B and the current sum:
+// the PLRC recursion and plrcStepD (fdtd_plrc.cpp:94-261, :304-427),
+// FDTD_Plain::stepD (fdtd_plain.cpp:37-77) or FDTD_Nonlinear::stepD
+// (fdtd_nl.cpp:38-100).  lc: the cell's medium coefficients (cell_coef, with
+// the conductivity already in them).  Counts a non-finite result in the status
+// word.
+template <typename T, int MODE, int NP, bool PLASMA>
+__device__ __forceinline__ void e_update(const EParams<T> &p, const CellCoef<T, NP> &lc, bool med, T ex, T ey, T ez,
+                                         T cbx, T cby, T cbz, T jx, T jy, T jz,
+                                         typename Vec2<T>::type (&q)[NP > 0 ? NP : 1][3], T &exn, T &eyn, T &ezn,
+                                         KerrCount &kc, const PlasmaCell<T> *pc) {
   const T dt = p.dt;
-  CellCoef<T, NP> lc;
-  cell_coef<T, NP, DESIGN>(p, i, j, k, med, lc);
-  if (PLASMA && med && p.pl_density) {
-    // numer - sig and denom + sig (fdtd_plrc.cpp:188-196, :356-359)
-    lc.numer = lc.numer - pc->sig;
-    lc.inv_denom = T(1) / (p.denom_t + pc->sig);
-    lc.inv_denom_lo = T(0);
-    lc.chi_over_denom = p.chi_raw / (p.denom_d + (double)pc->sig);
-  }
-  // ---- loads of the CPML psi of the faces containing the cell, and of the
-  // injection plane
-  T cp0[6], cp1[6], cb[6], cc[6];
-  int cli[6];  // layer arrays hold < 2^31 cells (checked by mp_create)
-  bool cin[6];
-#pragma unroll
-  for (int f = 0; f < 6; ++f) {
-    const CpmlFace<T> &F = p.cpml[f];
-    const int idx = face_axis(f) == 0 ? i + 1 : face_axis(f) == 1 ? j + 1 : k;
-    cin[f] = SPECIAL && (MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN) &&
-             (f < 4 ? ((cmask >> f) & 1u) != 0 : (F.active && k >= F.lo && k <= F.hi));
-    if (cin[f]) {
-      if (face_axis(f) == 2) cli[f] = ((k - F.lo) * p.ny + j) * p.nx + i;
-      else if (face_axis(f) == 0) cli[f] = ((k - F.zlo) * p.ny + j) * F.ex + (i + 1 - F.lo);
-      else cli[f] = ((k - F.zlo) * F.ey + (j + 1 - F.lo)) * p.nx + i;
-      cp0[f] = ld_c(F.psi0, cli[f], F.n, p.status);
-      cp1[f] = ld_c(F.psi1, cli[f], F.n, p.status);
-      cb[f] = ld(F.b + idx);
-      cc[f] = ld(F.c + idx);
-    }
-  }
-  T sa = T(0), sb = T(0);
-  bool on_src = false;
-  if (SPECIAL && (MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN)) {
-    for (int s = 0; s < p.n_src; ++s) {
-      if (k == p.src[s].plane) {
-        sa = ldg_c(p.src[s].v0, col, p.plane, p.status);
-        sb = ldg_c(p.src[s].v1, col, p.plane, p.status);
-        on_src = true;
-      }
-    }
-  }
-
-  // ---- E-side currents: CPML faces, then the injector plane
-  T jx = T(0), jy = T(0), jz = T(0);
-#pragma unroll
-  for (int f = 0; f < 6; ++f) {
-    if (!cin[f]) continue;
-    const int dim = face_axis(f);
-    T d0, d1;  // differences of B along dim for psi0, psi1
-    if (dim == 2) { d0 = -(v.by - v.by_km); d1 = v.bx - v.bx_km; }
-    else if (dim == 0) { d0 = -(v.bz - v.bz_xm); d1 = v.by - v.by_xm; }
-    else { d0 = -(v.bx - v.bx_ym); d1 = v.bz - v.bz_ym; }
-    cp0[f] = fma_pp(cb[f], cp0[f], cc[f], d0);
-    cp1[f] = fma_pp(cb[f], cp1[f], cc[f], d1);
-    if (dim == 2) { jx += cp0[f]; jy += cp1[f]; }
-    else if (dim == 0) { jy += cp0[f]; jz += cp1[f]; }
-    else { jz += cp0[f]; jx += cp1[f]; }
-  }
-  if (on_src) {
-    for (int m = 0; m < p.src_mult; ++m) {
-      jx += sa;
-      jy += sb;
-    }
-  }
-  if (PLASMA) {  // the plasma current, after the other currents
-    jx += pc->j[0];
-    jy += pc->j[1];
-    jz += pc->j[2];
-  }
-
-  // curl_kappa B (fdtd_plrc.cpp:207-244)
-  const T cbx = fma_pm(v.bz - v.bz_ym, iky, v.by - v.by_km, ikz);
-  const T cby = fma_pm(v.bx - v.bx_km, ikz, v.bz - v.bz_xm, ikx);
-  const T cbz = fma_pm(v.by - v.by_xm, ikx, v.bx - v.bx_ym, iky);
-  const T ex = v.ex, ey = v.ey, ez = v.ez;
-
   const T dtl = p.dt_lo;
   if (MODE == MODE_PLAIN) {
     exn = add_dt(ex, dt, dtl, cbx);
@@ -524,6 +461,85 @@ __device__ __forceinline__ void e_cell(const EParams<T> &p, int i, int j, int k,
     }
   }
   if (!finite3(exn, eyn, ezn)) atomicAdd(p.status + ST_NONFINITE, 1);
+}
+
+// SPECIAL = false: the caller guarantees that no CPML face contains the cell
+// and that k is no injection plane; the face and source code is left out.
+// PLASMA: *pc holds the plasma plug-ins' values of the cell (plasma_cell).
+template <typename T, int MODE, int NP, bool DESIGN = false, bool SPECIAL = true, bool PLASMA = false>
+__device__ __forceinline__ void e_cell(const EParams<T> &p, int i, int j, int k, long long col, bool med,
+                                       unsigned cmask, const EIn<T> &v, T ikx, T iky, T ikz,
+                                       typename Vec2<T>::type (&q)[NP > 0 ? NP : 1][3], T &exn, T &eyn,
+                                       T &ezn, KerrCount &kc, const PlasmaCell<T> *pc = nullptr) {
+  CellCoef<T, NP> lc;
+  cell_coef<T, NP, DESIGN>(p, i, j, k, med, lc);
+  if (PLASMA && med && p.pl_density) plasma_coef(p, pc->sig, lc);
+  // ---- loads of the CPML psi of the faces containing the cell, and of the
+  // injection plane
+  T cp0[6], cp1[6], cb[6], cc[6];
+  int cli[6];  // layer arrays hold < 2^31 cells (checked by mp_create)
+  bool cin[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const CpmlFace<T> &F = p.cpml[f];
+    const int idx = face_axis(f) == 0 ? i + 1 : face_axis(f) == 1 ? j + 1 : k;
+    cin[f] = SPECIAL && (MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN) &&
+             (f < 4 ? ((cmask >> f) & 1u) != 0 : (F.active && k >= F.lo && k <= F.hi));
+    if (cin[f]) {
+      if (face_axis(f) == 2) cli[f] = ((k - F.lo) * p.ny + j) * p.nx + i;
+      else if (face_axis(f) == 0) cli[f] = ((k - F.zlo) * p.ny + j) * F.ex + (i + 1 - F.lo);
+      else cli[f] = ((k - F.zlo) * F.ey + (j + 1 - F.lo)) * p.nx + i;
+      cp0[f] = ld_c(F.psi0, cli[f], F.n, p.status);
+      cp1[f] = ld_c(F.psi1, cli[f], F.n, p.status);
+      cb[f] = ld(F.b + idx);
+      cc[f] = ld(F.c + idx);
+    }
+  }
+  T sa = T(0), sb = T(0);
+  bool on_src = false;
+  if (SPECIAL && (MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN)) {
+    for (int s = 0; s < p.n_src; ++s) {
+      if (k == p.src[s].plane) {
+        sa = ldg_c(p.src[s].v0, col, p.plane, p.status);
+        sb = ldg_c(p.src[s].v1, col, p.plane, p.status);
+        on_src = true;
+      }
+    }
+  }
+
+  // ---- E-side currents: CPML faces, then the injector plane
+  T jx = T(0), jy = T(0), jz = T(0);
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    if (!cin[f]) continue;
+    const int dim = face_axis(f);
+    T d0, d1;  // differences of B along dim for psi0, psi1
+    if (dim == 2) { d0 = -(v.by - v.by_km); d1 = v.bx - v.bx_km; }
+    else if (dim == 0) { d0 = -(v.bz - v.bz_xm); d1 = v.by - v.by_xm; }
+    else { d0 = -(v.bx - v.bx_ym); d1 = v.bz - v.bz_ym; }
+    cp0[f] = fma_pp(cb[f], cp0[f], cc[f], d0);
+    cp1[f] = fma_pp(cb[f], cp1[f], cc[f], d1);
+    if (dim == 2) { jx += cp0[f]; jy += cp1[f]; }
+    else if (dim == 0) { jy += cp0[f]; jz += cp1[f]; }
+    else { jz += cp0[f]; jx += cp1[f]; }
+  }
+  if (on_src) {
+    for (int m = 0; m < p.src_mult; ++m) {
+      jx += sa;
+      jy += sb;
+    }
+  }
+  if (PLASMA) {  // the plasma current, after the other currents
+    jx += pc->j[0];
+    jy += pc->j[1];
+    jz += pc->j[2];
+  }
+
+  // curl_kappa B (fdtd_plrc.cpp:207-244)
+  const T cbx = fma_pm(v.bz - v.bz_ym, iky, v.by - v.by_km, ikz);
+  const T cby = fma_pm(v.bx - v.bx_km, ikz, v.bz - v.bz_xm, ikx);
+  const T cbz = fma_pm(v.by - v.by_xm, ikx, v.bx - v.bx_ym, iky);
+  e_update<T, MODE, NP, PLASMA>(p, lc, med, v.ex, v.ey, v.ez, cbx, cby, cbz, jx, jy, jz, q, exn, eyn, ezn, kc, pc);
   // ---- CPML stores
 #pragma unroll
   for (int f = 0; f < 6; ++f) {

@@ -129,6 +129,7 @@ struct EParams {
   // Newton iterations (accumulated; the sum over the slots counts)
   unsigned long long *kerr_count;
   long long n_field;      // elements of each field and history array
+  long long state_bytes;  // fields and PLRC accumulators
   long long n_psi;        // pairs of each PLRC accumulator array
 
   // Plasma plug-ins: PlasmaDensity (plasmadensity.cpp:18-49) and PlasmaCurrent
@@ -161,6 +162,7 @@ struct BParams {
   SourcePlane<T> src[4];
   int *status;
   long long n_field;      // elements of each field array
+  long long state_bytes;  // fields and PLRC accumulators
 };
 
 // ---------------------------------------------------------------------------

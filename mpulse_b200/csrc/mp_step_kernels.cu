@@ -1,6 +1,5 @@
 // mp_step_kernels.cu - the two half-step kernels of one MPulse time step,
-// global-load form (any grid size; mp_step_tma.cu has the TMA-staged form used
-// when the tile divides the grid).
+// global-load form (mp_step_tma.cu and mp_step_fused.cu hold two opt-in forms).
 //
 // e_half: FDTD_PLRCSolver::stepScheme's E side (fdtd_plrc.t:129-146) in one
 //   pass: the CPML psi_E recursions (CPMLBorderECurrent::stepScheme,
@@ -14,100 +13,205 @@
 //   (cpml_border.cpp:499-527), TF/SF M plane (incsource.t:112-145) and plrcStepB
 //   (fdtd_plrc.cpp:263-293).
 //
-// Thread mapping: one thread per (x, y) column, 32 x 4 columns per block; a
-// block marches up a chunk of z-planes so the z-neighbour of the previous plane
+// Thread mapping: V consecutive cells of a row per thread, the columns of a
+// plane dealt to warps as row_cells describes, whatever nx and ny are.  A block
+// marches up a chunk of z-planes, so that the z-neighbour of the previous plane
 // is carried in registers and every field element is read from HBM once per
-// half step (x/y neighbours are re-read through L1/L2).  The medium test, the
-// CPML z-faces and the source planes depend on z only and are uniform per
-// iteration.  The stencil has no contraction, so no tensor cores are involved;
-// both kernels are HBM-bandwidth bound.
+// half step (x/y neighbours are re-read through L1).  The medium test, the CPML
+// z-faces and the injection plane depend on z only and are uniform per plane.  A
+// plane's address is uniform too: each access is that address plus a 32-bit
+// column offset fixed through the march.
+//
+// What bounds them.  The stencil has no contraction, so no tensor cores.  On
+// grids that exceed L2 both kernels are bound by HBM, on smaller ones by the
+// instructions they issue (before this form 541 per 32 cells in the E half and
+// 394 in the B half of a 96^3 grid with CPML on all faces, issue slots 68% and
+// 60% busy; now 387 and 257), which is why the faces are found from six
+// thresholds, rows from a multiplication, and nothing is tested per cell that is
+// fixed per thread or per plane.  On large grids the loads of one plane per
+// warp do not cover the latency of HBM: the next plane's lines are prefetched
+// into L2 while this plane is computed, which needs no registers.
+// Measured per half step, before -> after (B200, us):
+//   256 x 256 x 512 PLRC + Kerr FP32   E 758 -> 681   B 276 -> 258
+//   192 x 192 x 384 PLRC + Kerr FP64   E 659 -> 551   B 225 -> 198
+//   150 x 131 x 210 fdtd-plain FP32    E  37 ->  30   B  48 ->  31
+//   101 x 75 x 163 fdtd-nl FP64        E  49 ->  26   B  40 ->  17
+//   128 x 128 x 192 + plasma FP32      E 135 -> 109   B  56 ->  43
 #include "mp_cell.cuh"
 
 #include <algorithm>
 
-// Block shape 32 x BLOCK_Y columns (a warp is one row of 32 columns) and the
-// minimum resident threads per SM asked of the register allocator, 768 (80
-// registers).  Measured on the 256x256x512 PLRC + Kerr workload (FP32), with
-// 32 x 8 blocks: E half 1.083 ms with no bound (114 registers), 0.917 ms with
-// 768 threads (80 registers, 28 B spilled), 1.17 ms with 1024 (64 registers,
-// more spills); 32 x 4 blocks then took the E half from 0.872 to 0.859 ms and
-// the B half from 0.462 to 0.440 ms (32 x 2: no further gain).
-#ifndef MPB_E_BLOCK_Y
-#define MPB_E_BLOCK_Y 4
+// Resident threads per SM asked of the register allocator.  E half: FP32 with
+// one cell per thread 1024 (64 registers; 768 lets the compiler take 75 with the
+// plasma plug-ins: 114 instead of 109 us on 128 x 128 x 192), with two cells 768
+// (80 registers); FP64 640 (96 registers; 768 spill: 96 instead of 87 us with a
+// design region, 120 x 104 x 136).  B half: FP32 1280 (48 registers; 1024: 264
+// instead of 257 us on 256 x 256 x 512), FP64 768 (640: 205, 1024: 206, 768:
+// 198 us on 192 x 192 x 384).
+#ifndef MPB_E_THREADS_F
+#define MPB_E_THREADS_F 1024
 #endif
-#ifndef MPB_B_BLOCK_Y
-#define MPB_B_BLOCK_Y 4
+#ifndef MPB_E_THREADS_F2
+#define MPB_E_THREADS_F2 768
 #endif
-#ifndef MPB_E_MIN_THREADS
-#define MPB_E_MIN_THREADS 768
+#ifndef MPB_E_THREADS_D
+#define MPB_E_THREADS_D 640
 #endif
-// FP32 E half: resident threads per SM (the FP64 form keeps MPB_E_MIN_THREADS).
-// On the 256x256x512 workload with the pulse in the Kerr medium (FP32, where
-// the E half is latency- and issue-bound) 1024 threads (64 registers, 40 B
-// spilled) took the E half from 0.855 to 0.839 ms.
-#ifndef MPB_E_MIN_THREADS_F
-#define MPB_E_MIN_THREADS_F 1024
+#ifndef MPB_B_THREADS_F
+#define MPB_B_THREADS_F 1280
 #endif
-#ifndef MPB_B_MIN_THREADS
-#define MPB_B_MIN_THREADS 768
-#endif
-// E half z-chunks: planes per block chosen for about this many blocks of
-// 32 x MPB_E_BLOCK_Y columns per SM, so that the last, partly filled wave of
-// blocks is a small part of the launch, and at least MPB_E_MIN_PLANES planes
-// per block (the z-march carries the plane below in registers).  Measured on
-// the 256x256x512 PLRC + Kerr workload with the pulse in the Kerr medium
-// (FP32, E half): 103 planes per block (2560 blocks, 2.2 waves of the 1184
-// resident) 0.847 ms, 47 / 32 / 23 / 16 / 8 planes 0.774 / 0.772 / 0.757 /
-// 0.769 / 0.774 ms; blocks per SM 64 / 80 / 112: 0.765 / 0.758 / 0.753 ms.
-// FP64 (768 resident threads), 103 planes 1.695 ms, 24 / 48 / 80 blocks per
-// SM 1.632 / 1.563 / 1.540 ms.  On the 96^3 adjoint workload the forward run
-// takes the same time with at least 1, 2, 4 or 8 planes per block (±3%).
-#ifndef MPB_E_BLOCKS_PER_SM_F
-#define MPB_E_BLOCKS_PER_SM_F 80
-#endif
-#ifndef MPB_E_BLOCKS_PER_SM_D
-#define MPB_E_BLOCKS_PER_SM_D 80
-#endif
-#ifndef MPB_E_MIN_PLANES
-#define MPB_E_MIN_PLANES 2
-#endif
-// B half: two cells per thread with vector loads along x where nx allows,
-// with its own occupancy and z-chunks (half the threads), per precision.
-// Measured on the 256x256x512 workload (FP32, B half): scalar kernel 0.440
-// ms; four cells per thread (float4), 768 threads, chunks for 24 blocks per SM
-// 0.354 ms; two cells per thread (float2) with 768 / 1024 / 1280 / 1536
-// threads 0.335 / 0.293 / 0.304 / 0.302 ms, 1024 threads and 32 / 48 blocks
-// per SM 0.290 / 0.285 ms (32 x 2 blocks: 0.284 ms, 32 x 8: 0.307 ms).  FP64 (double2), B half with 512 / 640 / 768 / 1024 threads:
-// 0.553 / 0.488 / 0.538 / 0.560 ms.  Re-measured with the pulse in the Kerr
-// medium and the E half's z-chunks for 80 blocks per SM: FP32 48 / 80 / 128
-// blocks per SM 0.295 / 0.281 / 0.286 ms, FP64 24 / 48 / 80 blocks per SM
-// 0.510 / 0.495 / 0.468 ms; at least 4 instead of 8 planes per block: no
-// change.
-#ifndef MPB_B_VECTOR
-#define MPB_B_VECTOR 1
-#endif
-#ifndef MPB_BV_MIN_THREADS_F
-#define MPB_BV_MIN_THREADS_F 1024
-#endif
-#ifndef MPB_BV_MIN_THREADS_D
-#define MPB_BV_MIN_THREADS_D 640
-#endif
-#ifndef MPB_BV_BLOCKS_PER_SM_F
-#define MPB_BV_BLOCKS_PER_SM_F 80
-#endif
-#ifndef MPB_BV_BLOCKS_PER_SM_D
-#define MPB_BV_BLOCKS_PER_SM_D 80
-#endif
-#ifndef MPB_BV_MIN_PLANES
-#define MPB_BV_MIN_PLANES 8
-#endif
-// B half, scalar kernel: issue the next plane's loads before the current
-// plane's arithmetic.
-#ifndef MPB_B_PREFETCH
-#define MPB_B_PREFETCH 1
+#ifndef MPB_B_THREADS_D
+#define MPB_B_THREADS_D 768
 #endif
 
 namespace mpb {
+
+// Rows (warps) per block: with one row the y neighbours come from other blocks
+// through L2 and the 256 x 256 x 512 E half takes 824 instead of 737 us; 2 and 8
+// rows 1% and 7% slower than 4.
+constexpr int kRowTile = 4;
+constexpr int kRowThreads = 32 * kRowTile;
+
+// Programmatic dependent launch: let the next kernel of the stream start its
+// blocks once all of this kernel's have started, and wait for the previous
+// kernel's writes.  Both are no-ops for a kernel launched without the attribute.
+// Every kernel of a chain waits, so the end of one is the end of all before it.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
+
+// V consecutive elements of a row.
+template <typename T, int V>
+struct alignas(sizeof(T) * V <= 16 ? sizeof(T) * V : 16) RowV {
+  T v[V];
+};
+
+// The accesses at column c of the plane at element `base` of an array of n
+// elements (aligned to a row of V), checked like ld_c / st_c.  Plain loads, not
+// the read-only path: a kernel launched early must not have them moved ahead
+// of its wait.
+template <typename T, int V>
+__device__ __forceinline__ bool row_in(long long i, long long n, int *st) {
+  return in_bounds(i, n, st) && (V == 1 || in_bounds(i + V - 1, n, st));
+}
+template <int V, typename T>
+__device__ __forceinline__ RowV<T, V> ldp(const T *a, long long base, unsigned c, long long n, int *st) {
+  RowV<T, V> r = {};
+  if (row_in<T, V>(base + c, n, st)) r = *reinterpret_cast<const RowV<T, V> *>(a + base + c);
+  return r;
+}
+template <int V, typename T>
+__device__ __forceinline__ void stp(T *a, long long base, unsigned c, long long n, int *st, const RowV<T, V> &r) {
+  if (row_in<T, V>(base + c, n, st)) *reinterpret_cast<RowV<T, V> *>(a + base + c) = r;
+}
+
+// The columns of a thread, row j, columns i0 .. i0 + V - 1 of the plane: rows
+// are taken in groups of kRowTile, warp w of a block holds row w of a group, and
+// its 32 lanes run along the row and on into the same row of the next group, so
+// that a block covers kRowTile neighbouring rows (their y neighbours meet in
+// L1) and no lane is idle on narrow or odd rows.
+struct RowGrid {
+  unsigned nrow, nvec;  // threads per row (nx / V), and per warp over all groups
+  unsigned mul, shift;  // t / nrow = (t * mul) >> (32 + shift) for t < 2^31
+  int kchunk;           // planes per block
+  int ahead;            // prefetch the next plane into L2
+  // the CPML layers: cells with MPulse index <= lo[a] or >= hi[a] along axis a
+  // lie in a layer
+  int lo[3], hi[3];
+  int src;              // the injection plane (-1: none)
+};
+
+template <int V>
+__device__ __forceinline__ bool row_cells(const RowGrid &g, int ny, int &i0, int &j) {
+  const unsigned t = blockIdx.x * 32 + (threadIdx.x & 31);
+  const unsigned grp = __umulhi(t, g.mul) >> g.shift;
+  i0 = int(t - grp * g.nrow) * V;
+  j = int(grp * kRowTile + (threadIdx.x >> 5));
+  return t < g.nvec && j < ny;
+}
+
+// Bits of the x faces (slots 2 high, 3 low) at the V cells of a thread, bits 2c
+// and 2c + 1, and of the y faces (slots 0 high, 1 low), bits 2V and 2V + 1.
+template <int V>
+__device__ __forceinline__ unsigned row_face_mask(const RowGrid &g, int i0, int j) {
+  unsigned m = (j + 1 >= g.hi[1] ? 1u << (2 * V) : 0u) | (j + 1 <= g.lo[1] ? 2u << (2 * V) : 0u);
+#pragma unroll
+  for (int c = 0; c < V; ++c)
+    m |= (i0 + c + 1 >= g.hi[0] ? 1u << (2 * c) : 0u) | (i0 + c + 1 <= g.lo[0] ? 2u << (2 * c) : 0u);
+  return m;
+}
+
+// One CPML face over the V cells of a thread at plane k: psi <- b psi + c d
+// for both components, the new psi stored and added to the two current
+// components the face feeds (x faces y and z, y faces z and x, z faces x and
+// y).  d0, d1: the differences along the face's axis.  ONE: only cell c0 (x
+// faces, whose layers begin and end inside a row).
+template <typename T, int V, int F>
+__device__ __forceinline__ void face_row(const CpmlFace<T> &L, int nx, int ny, int i0, int j, int k, int c0,
+                                         const T (&d0)[V], const T (&d1)[V], T (&cur)[V][3], int *st) {
+  constexpr int dim = face_axis(F);
+  constexpr int u = (dim + 1) % 3, w = (dim + 2) % 3;
+  if (dim == 0) {
+    const int li = ((k - L.zlo) * ny + j) * L.ex + (i0 + c0 + 1 - L.lo);
+    const T b = ld(L.b + i0 + c0 + 1), c = ld(L.c + i0 + c0 + 1);
+    const T p0 = fma_pp(b, ld_c(L.psi0, li, L.n, st), c, d0[c0]);
+    const T p1 = fma_pp(b, ld_c(L.psi1, li, L.n, st), c, d1[c0]);
+    st_c(L.psi0, li, L.n, st, p0);
+    st_c(L.psi1, li, L.n, st, p1);
+    cur[c0][u] += p0;
+    cur[c0][w] += p1;
+  } else {
+    const int idx = dim == 1 ? j + 1 : k;
+    const unsigned li = dim == 1 ? unsigned(((k - L.zlo) * L.ey + (j + 1 - L.lo)) * nx + i0)
+                                 : unsigned(((k - L.lo) * ny + j) * nx + i0);
+    const T b = ld(L.b + idx), c = ld(L.c + idx);
+    RowV<T, V> p0 = ldp<V>(L.psi0, 0, li, L.n, st), p1 = ldp<V>(L.psi1, 0, li, L.n, st);
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      p0.v[q] = fma_pp(b, p0.v[q], c, d0[q]);
+      p1.v[q] = fma_pp(b, p1.v[q], c, d1[q]);
+      cur[q][u] += p0.v[q];
+      cur[q][w] += p1.v[q];
+    }
+    stp<V>(L.psi0, 0, li, L.n, st, p0);
+    stp<V>(L.psi1, 0, li, L.n, st, p1);
+  }
+}
+
+// All faces containing the cells of a thread, in MPulse's order (slots 0..5):
+// the differences along y, x and z of the components the faces take, with the
+// sign of the side.
+template <typename T, int V>
+__device__ __forceinline__ void face_currents(const CpmlFace<T> (&cpml)[6], int nx, int ny, unsigned mask, bool zlow,
+                                              bool zhigh, int i0, int j, int k, const T (&dy0)[V], const T (&dy1)[V],
+                                              const T (&dx0)[V], const T (&dx1)[V], const T (&dz0)[V],
+                                              const T (&dz1)[V], T (&cur)[V][3], int *st) {
+  if (mask) {
+    if (mask & (1u << (2 * V))) face_row<T, V, 0>(cpml[0], nx, ny, i0, j, k, 0, dy0, dy1, cur, st);
+    if (mask & (2u << (2 * V))) face_row<T, V, 1>(cpml[1], nx, ny, i0, j, k, 0, dy0, dy1, cur, st);
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      if (mask & (1u << (2 * c))) face_row<T, V, 2>(cpml[2], nx, ny, i0, j, k, c, dx0, dx1, cur, st);
+      if (mask & (2u << (2 * c))) face_row<T, V, 3>(cpml[3], nx, ny, i0, j, k, c, dx0, dx1, cur, st);
+    }
+  }
+  if (zhigh) face_row<T, V, 4>(cpml[4], nx, ny, i0, j, k, 0, dz0, dz1, cur, st);
+  if (zlow) face_row<T, V, 5>(cpml[5], nx, ny, i0, j, k, 0, dz0, dz1, cur, st);
+}
+
+// The injection plane's currents of the V cells.
+template <typename T, int V, typename P>
+__device__ __forceinline__ void source_currents(const P &p, unsigned col, T (&cur)[V][3]) {
+  const RowV<T, V> a = ldp<V>(p.src[0].v0, 0, col, p.plane, p.status);
+  const RowV<T, V> b = ldp<V>(p.src[0].v1, 0, col, p.plane, p.status);
+#pragma unroll
+  for (int c = 0; c < V; ++c)
+    for (int q = 0; q < p.src_mult; ++q) {
+      cur[c][0] += a.v[c];
+      cur[c][1] += b.v[c];
+    }
+}
 
 // Whether the adjoint history of cell (i, j, k) is stored (EParams::hist_box).
 template <typename T>
@@ -121,400 +225,268 @@ __device__ __forceinline__ bool hist_cell(const EParams<T> &p, int i, int j, int
   return false;
 }
 
-template <typename T, int MODE, int NP, bool DESIGN, bool PLASMA = false>
-__global__ void __launch_bounds__(32 * MPB_E_BLOCK_Y,
-                                  (sizeof(T) == 4 ? MPB_E_MIN_THREADS_F : MPB_E_MIN_THREADS) / (32 * MPB_E_BLOCK_Y))
-    e_half_kernel(const EParams<T> p) {
+template <typename T, int V, int MODE, int NP, bool DESIGN, bool PLASMA>
+__global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 8 ? MPB_E_THREADS_D : V == 1 ? MPB_E_THREADS_F : MPB_E_THREADS_F2) / kRowThreads)
+    e_half_kernel(const EParams<T> p, const RowGrid g) {
   typedef typename Vec2<T>::type T2;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // 0-based: MPulse i + 1
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= p.nx || j >= p.ny) return;
-  const int k0 = p.k_first + blockIdx.z * p.kchunk;
-  const int k1 = min(k0 + p.kchunk - 1, p.k_last);
-  if (k0 > k1) return;
-
+  constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
+  pdl_launch_dependents();
+  const int nx = p.nx, ny = p.ny;
+  int i0, j;  // 0-based: MPulse i + 1, j + 1
+  if (!row_cells<V>(g, ny, i0, j)) return;
+  const int k0 = p.k_first + blockIdx.y * g.kchunk;
+  const int k1 = min(k0 + g.kchunk - 1, p.k_last);
   const long long plane = p.plane;
-  const int im = (i == 0) ? p.nx - 1 : i - 1;
-  const int jm = (j == 0) ? p.ny - 1 : j - 1;
-  const long long col = (long long)j * p.nx + i;
-  const long long colxm = (long long)j * p.nx + im;
-  const long long colym = (long long)jm * p.nx + i;
-  const T *__restrict__ Bx = p.B[0];
-  const T *__restrict__ By = p.B[1];
-  const T *__restrict__ Bz = p.B[2];
-  T *__restrict__ Ex = p.E[0];
-  T *__restrict__ Ey = p.E[1];
-  T *__restrict__ Ez = p.E[2];
-  const T ikx = ld(p.ik[0] + i + 1);
+  const unsigned row = unsigned(j) * unsigned(nx);
+  const unsigned col = row + i0;
+  const unsigned colxm = row + (i0 == 0 ? nx - 1 : i0 - 1);  // x-1 of the first cell
+  const unsigned colym = (j == 0 ? unsigned(plane) : row) - nx + i0;
+  const T *Bx = p.B[0], *By = p.B[1], *Bz = p.B[2];
+  T *Ex = p.E[0], *Ey = p.E[1], *Ez = p.E[2];
+  RowV<T, V> ikx;
+#pragma unroll
+  for (int c = 0; c < V; ++c) ikx.v[c] = ld(p.ik[0] + i0 + c + 1);
   const T iky = ld(p.ik[1] + j + 1);
-  // CPML faces: the x / y faces of this warp's columns are fixed through the
-  // z-march; warps with none skip the face code on planes outside the z faces
-  const unsigned cmask = face_column_mask(p.cpml, i, j);
-  const bool warp_xy = __any_sync(__activemask(), cmask != 0u);
-  const int2 srck = source_plane_range(p);
-
-  int km = k0 - 1;
-  if (p.zperiodic && km == 0) km = p.nz;
+  const unsigned fmask = PLRC ? row_face_mask<V>(g, i0, j) : 0u;
   const long long nf = p.n_field;
   int *const st = p.status;
-  T bx_km = ldg_c(Bx, km * plane + col, nf, st);
-  T by_km = ldg_c(By, km * plane + col, nf, st);
   KerrCount kc;
+  pdl_wait();
 
+  const int km = p.zperiodic && k0 == 1 ? p.nz : k0 - 1;
+  RowV<T, V> bx_km = ldp<V>(Bx, km * plane, col, nf, st), by_km = ldp<V>(By, km * plane, col, nf, st);
   for (int k = k0; k <= k1; ++k) {
     const long long base = (long long)k * plane;
-    // ---- loads of this cell (the rest are in e_cell, still before any store)
-    EIn<T> v;
-    v.bx = ldg_c(Bx, base + col, nf, st);
-    v.by = ldg_c(By, base + col, nf, st);
-    v.bz = ldg_c(Bz, base + col, nf, st);
-    v.bz_xm = ldg_c(Bz, base + colxm, nf, st);
-    v.by_xm = ldg_c(By, base + colxm, nf, st);
-    v.bz_ym = ldg_c(Bz, base + colym, nf, st);
-    v.bx_ym = ldg_c(Bx, base + colym, nf, st);
-    v.bx_km = bx_km;
-    v.by_km = by_km;
-    v.ex = ld_c(Ex, base + col, nf, st);
-    v.ey = ld_c(Ey, base + col, nf, st);
-    v.ez = ld_c(Ez, base + col, nf, st);
+    // ---- every load of this plane first
+    const RowV<T, V> bx = ldp<V>(Bx, base, col, nf, st), by = ldp<V>(By, base, col, nf, st),
+                     bz = ldp<V>(Bz, base, col, nf, st);
+    const RowV<T, V> bz_ym = ldp<V>(Bz, base, colym, nf, st), bx_ym = ldp<V>(Bx, base, colym, nf, st);
+    const RowV<T, 1> bz_xl = ldp<1>(Bz, base, colxm, nf, st), by_xl = ldp<1>(By, base, colxm, nf, st);
+    const RowV<T, V> ex = ldp<V>(Ex, base, col, nf, st), ey = ldp<V>(Ey, base, col, nf, st),
+                     ez = ldp<V>(Ez, base, col, nf, st);
+    const bool med = PLRC && k >= p.mz0 && k <= p.mz1;
+    const long long pbase = (long long)(k - p.mz0) * plane;
+    RowV<T2, V> q[NP > 0 ? NP : 1][3];
+    if (NP > 0 && med) {
+#pragma unroll
+      for (int n = 0; n < NP; ++n)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          q[n][c] = ldp<V>(reinterpret_cast<const T2 *>(p.psi[n][c]), pbase, col, p.n_psi, st);
+    }
+    RowV<T, V> rho, j0 = {}, j1 = {}, j2 = {};
+    if (PLASMA) {
+      rho = ldp<V>(p.rho, base, col, nf, st);
+      if (p.pl_current) {
+        j0 = ldp<V>(p.pj[0], base, col, nf, st);
+        j1 = ldp<V>(p.pj[1], base, col, nf, st);
+        j2 = ldp<V>(p.pj[2], base, col, nf, st);
+      }
+    }
     const T ikz = ld(p.ik[2] + k);
-    const bool med = (MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN) && k >= p.mz0 && k <= p.mz1;
-    const long long pi = ((long long)(k - p.mz0) * p.ny + j) * p.nx + i;
-    T2 q[NP > 0 ? NP : 1][3];
-    if (NP > 0 && med) {
+    if (g.ahead && k < k1) {
+      const long long ba = base + plane;
+      prefetch_l2(Bx + ba + col);
+      prefetch_l2(By + ba + col);
+      prefetch_l2(Bz + ba + col);
+      prefetch_l2(Ex + ba + col);
+      prefetch_l2(Ey + ba + col);
+      prefetch_l2(Ez + ba + col);
+      if (NP > 0 && med) {
+#pragma unroll
+        for (int n = 0; n < NP; ++n)
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            prefetch_l2(reinterpret_cast<const T2 *>(p.psi[n][c]) + pbase + plane + col);
+      }
+    }
+
+    // ---- the differences of B, then the E-side currents in MPulse's order
+    T dzy[V], dyz[V], dxz[V], dzx[V], dyx[V], dxy[V];  // d<component><axis>
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      dzy[c] = bz.v[c] - bz_ym.v[c];
+      dxy[c] = bx.v[c] - bx_ym.v[c];
+      dzx[c] = bz.v[c] - (c ? bz.v[c ? c - 1 : 0] : bz_xl.v[0]);
+      dyx[c] = by.v[c] - (c ? by.v[c ? c - 1 : 0] : by_xl.v[0]);
+      dxz[c] = bx.v[c] - bx_km.v[c];
+      dyz[c] = by.v[c] - by_km.v[c];
+    }
+    T cur[V][3];
+#pragma unroll
+    for (int c = 0; c < V; ++c) cur[c][0] = cur[c][1] = cur[c][2] = T(0);
+    if (PLRC) {
+      const bool zlow = k <= g.lo[2], zhigh = k >= g.hi[2];
+      if (fmask || zlow || zhigh) {
+        T nxy[V], nzx[V], nyz[V];
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+          nxy[c] = -dxy[c];
+          nzx[c] = -dzx[c];
+          nyz[c] = -dyz[c];
+        }
+        face_currents<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, nxy, dzy, nzx, dyx, nyz, dxz, cur, st);
+      }
+      if (k == g.src) source_currents<T, V>(p, col, cur);
+    }
+
+    // ---- the E update, cell by cell
+    RowV<T, V> exn, eyn, ezn;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      CellCoef<T, NP> lc;
+      cell_coef<T, NP, DESIGN>(p, i0 + c, j, k, med, lc);
+      PlasmaCell<T> pc;
+      if (PLASMA) {
+        plasma_cell(p, ex.v[c], ey.v[c], ez.v[c], rho.v[c], j0.v[c], j1.v[c], j2.v[c], pc);
+        if (med && p.pl_density) plasma_coef(p, pc.sig, lc);
+        rho.v[c] = pc.rho;
+        j0.v[c] = pc.j[0];
+        j1.v[c] = pc.j[1];
+        j2.v[c] = pc.j[2];
+        // the plasma current, after the other currents
+        cur[c][0] += pc.j[0];
+        cur[c][1] += pc.j[1];
+        cur[c][2] += pc.j[2];
+      }
+      // curl_kappa B (fdtd_plrc.cpp:207-244)
+      const T cbx = fma_pm(dzy[c], iky, dyz[c], ikz);
+      const T cby = fma_pm(dxz[c], ikz, dzx[c], ikx.v[c]);
+      const T cbz = fma_pm(dyx[c], ikx.v[c], dxy[c], iky);
+      T2 qc[NP > 0 ? NP : 1][3];
 #pragma unroll
       for (int n = 0; n < NP; ++n)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) q[n][c] = ld_c(reinterpret_cast<const T2 *>(p.psi[n][c]), pi, p.n_psi, st);
+        for (int a = 0; a < 3; ++a) qc[n][a] = q[n][a].v[c];
+      e_update<T, MODE, NP, PLASMA>(p, lc, med, ex.v[c], ey.v[c], ez.v[c], cbx, cby, cbz, cur[c][0], cur[c][1],
+                                    cur[c][2], qc, exn.v[c], eyn.v[c], ezn.v[c], kc, &pc);
+#pragma unroll
+      for (int n = 0; n < NP; ++n)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) q[n][a].v[c] = qc[n][a];
     }
-    PlasmaCell<T> pc;
-    if (PLASMA) {
-      const T r0 = ld_c(p.rho, base + col, nf, st);
-      T j0 = T(0), j1 = T(0), j2 = T(0);
-      if (p.pl_current) {
-        j0 = ld_c(p.pj[0], base + col, nf, st);
-        j1 = ld_c(p.pj[1], base + col, nf, st);
-        j2 = ld_c(p.pj[2], base + col, nf, st);
-      }
-      plasma_cell(p, v.ex, v.ey, v.ez, r0, j0, j1, j2, pc);
-    }
-    T exn, eyn, ezn;
-    if (warp_xy || z_face_plane(p.cpml, k) || (k >= srck.x && k <= srck.y))
-      e_cell<T, MODE, NP, DESIGN, true, PLASMA>(p, i, j, k, col, med, cmask, v, ikx, iky, ikz, q, exn, eyn, ezn, kc,
-                                                &pc);
-    else
-      e_cell<T, MODE, NP, DESIGN, false, PLASMA>(p, i, j, k, col, med, cmask, v, ikx, iky, ikz, q, exn, eyn, ezn,
-                                                 kc, &pc);
     // ---- stores
-    st_c(Ex, base + col, nf, st, exn);
-    st_c(Ey, base + col, nf, st, eyn);
-    st_c(Ez, base + col, nf, st, ezn);
+    stp<V>(Ex, base, col, nf, st, exn);
+    stp<V>(Ey, base, col, nf, st, eyn);
+    stp<V>(Ez, base, col, nf, st, ezn);
     if (PLASMA) {
-      st_c(p.rho, base + col, nf, st, pc.rho);
+      stp<V>(p.rho, base, col, nf, st, rho);
       if (p.pl_current) {
-        st_c(p.pj[0], base + col, nf, st, pc.j[0]);
-        st_c(p.pj[1], base + col, nf, st, pc.j[1]);
-        st_c(p.pj[2], base + col, nf, st, pc.j[2]);
+        stp<V>(p.pj[0], base, col, nf, st, j0);
+        stp<V>(p.pj[1], base, col, nf, st, j1);
+        stp<V>(p.pj[2], base, col, nf, st, j2);
       }
     }
-    if (DESIGN && p.hist[0] && hist_cell(p, i, j, k)) {
-      st_c(p.hist[0], base + col, nf, st, exn);
-      st_c(p.hist[1], base + col, nf, st, eyn);
-      st_c(p.hist[2], base + col, nf, st, ezn);
+    if (DESIGN && p.hist[0]) {
+#pragma unroll
+      for (int c = 0; c < V; ++c)
+        if (hist_cell(p, i0 + c, j, k)) {
+          st_c(p.hist[0], base + col + c, nf, st, exn.v[c]);
+          st_c(p.hist[1], base + col + c, nf, st, eyn.v[c]);
+          st_c(p.hist[2], base + col + c, nf, st, ezn.v[c]);
+        }
     }
     if (NP > 0 && med) {
 #pragma unroll
       for (int n = 0; n < NP; ++n)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) st_c(reinterpret_cast<T2 *>(p.psi[n][c]), pi, p.n_psi, st, q[n][c]);
+        for (int c = 0; c < 3; ++c) stp<V>(reinterpret_cast<T2 *>(p.psi[n][c]), pbase, col, p.n_psi, st, q[n][c]);
     }
-    bx_km = v.bx;
-    by_km = v.by;
+    bx_km = bx;
+    by_km = by;
   }
   flush_kerr_count<MODE>(p.kerr_count, kc);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(32 * MPB_B_BLOCK_Y, MPB_B_MIN_THREADS / (32 * MPB_B_BLOCK_Y))
-    b_half_kernel(const BParams<T> p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= p.nx || j >= p.ny) return;
-  const int k0 = p.k_first + blockIdx.z * p.kchunk;
-  const int k1 = min(k0 + p.kchunk - 1, p.k_last);
-  if (k0 > k1) return;
-
+template <typename T, int V>
+__global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F : MPB_B_THREADS_D) / kRowThreads)
+    b_half_kernel(const BParams<T> p, const RowGrid g) {
+  // the chunks from the top down: the E half wrote the top planes last, and
+  // what of them is still in L2 is read from there (2-6% of both halves on grids
+  // of up to twice the L2)
+  pdl_launch_dependents();
+  const int nx = p.nx, ny = p.ny;
+  int i0, j;
+  if (!row_cells<V>(g, ny, i0, j)) return;
+  const int k0 = p.k_first + (gridDim.y - 1 - blockIdx.y) * g.kchunk;
+  const int k1 = min(k0 + g.kchunk - 1, p.k_last);
   const long long plane = p.plane;
-  const int ip = (i == p.nx - 1) ? 0 : i + 1;
-  const int jp = (j == p.ny - 1) ? 0 : j + 1;
-  const long long col = (long long)j * p.nx + i;
-  const long long colxp = (long long)j * p.nx + ip;
-  const long long colyp = (long long)jp * p.nx + i;
-  const T *__restrict__ Ex = p.E[0];
-  const T *__restrict__ Ey = p.E[1];
-  const T *__restrict__ Ez = p.E[2];
-  T *__restrict__ Bx = p.B[0];
-  T *__restrict__ By = p.B[1];
-  T *__restrict__ Bz = p.B[2];
-  const T ikx = ld(p.ik[0] + i + 1);
+  const unsigned row = unsigned(j) * unsigned(nx);
+  const unsigned col = row + i0;
+  const unsigned colxp = row + (i0 + V == nx ? 0 : i0 + V);  // x+1 of the last cell
+  const unsigned colyp = (j == ny - 1 ? 0u : row + nx) + i0;
+  const T *Ex = p.E[0], *Ey = p.E[1], *Ez = p.E[2];
+  T *Bx = p.B[0], *By = p.B[1], *Bz = p.B[2];
+  RowV<T, V> ikx;
+#pragma unroll
+  for (int c = 0; c < V; ++c) ikx.v[c] = ld(p.ik[0] + i0 + c + 1);
   const T iky = ld(p.ik[1] + j + 1);
   const T iky_bz = ld(p.ik_bz_y + j + 1);
-  const unsigned cmask = face_column_mask(p.cpml, i, j);
-  const bool warp_xy = __any_sync(__activemask(), cmask != 0u);
-  const int2 srck = source_plane_range(p);
-
-  // loads of plane k (ex, ey of plane k are carried from the previous plane)
+  const unsigned fmask = row_face_mask<V>(g, i0, j);
   const long long nf = p.n_field;
   int *const st = p.status;
-  auto load = [&](int k, T ex_k, T ey_k, BIn<T> &v) {
-    const long long base = (long long)k * plane;
-    int kp = k + 1;
-    if (p.zperiodic && kp == p.nz + 1) kp = 1;
-    const long long basep = (long long)kp * plane;
-    v.ex = ex_k;
-    v.ey = ey_k;
-    v.ex_kp = ldg_c(Ex, basep + col, nf, st);
-    v.ey_kp = ldg_c(Ey, basep + col, nf, st);
-    v.ez = ldg_c(Ez, base + col, nf, st);
-    v.ez_xp = ldg_c(Ez, base + colxp, nf, st);
-    v.ey_xp = ldg_c(Ey, base + colxp, nf, st);
-    v.ez_yp = ldg_c(Ez, base + colyp, nf, st);
-    v.ex_yp = ldg_c(Ex, base + colyp, nf, st);
-    v.bx = ld_c(Bx, base + col, nf, st);
-    v.by = ld_c(By, base + col, nf, st);
-    v.bz = ld_c(Bz, base + col, nf, st);
-  };
+  pdl_wait();
 
-  BIn<T> v;
-  load(k0, ldg_c(Ex, (long long)k0 * plane + col, nf, st), ldg_c(Ey, (long long)k0 * plane + col, nf, st), v);
+  RowV<T, V> ex = ldp<V>(Ex, k0 * plane, col, nf, st), ey = ldp<V>(Ey, k0 * plane, col, nf, st);
   for (int k = k0; k <= k1; ++k) {
     const long long base = (long long)k * plane;
-#if MPB_B_PREFETCH
-    // the next plane's loads go out before this plane's arithmetic and stores
-    // (they never alias them: B of plane k+1, E is read-only here)
-    BIn<T> vn;
-    if (k < k1) load(k + 1, v.ex_kp, v.ey_kp, vn);
-#endif
-    const T ikz = ld(p.ik[2] + k);
-    T bxn, byn, bzn;
-    if (warp_xy || z_face_plane(p.cpml, k) || (k >= srck.x && k <= srck.y))
-      b_cell<T, true>(p, i, j, k, col, cmask, v, ikx, iky, iky_bz, ikz, bxn, byn, bzn);
-    else
-      b_cell<T, false>(p, i, j, k, col, cmask, v, ikx, iky, iky_bz, ikz, bxn, byn, bzn);
-    st_c(Bx, base + col, nf, st, bxn);
-    st_c(By, base + col, nf, st, byn);
-    st_c(Bz, base + col, nf, st, bzn);
-#if MPB_B_PREFETCH
-    v = vn;
-#else
-    if (k < k1) load(k + 1, v.ex_kp, v.ey_kp, v);
-#endif
-  }
-}
-
-// The B half with vector loads along x: each thread owns V = 2 consecutive
-// cells of a row (nx a multiple of 64), so a plane's loads are 8 float2 /
-// double2 vectors and two scalars (the x+1 neighbour of the second cell), and
-// the z+1 plane of E is carried to the next plane.  The CPML faces add their
-// currents cell by cell (y faces hold whole rows, x faces single cells, z
-// faces whole planes).
-template <typename T> struct VecB;
-template <> struct VecB<float> { typedef float2 type; };
-template <> struct VecB<double> { typedef double2 type; };
-constexpr int kBV = 2;  // cells per thread
-
-template <typename T>
-struct RowV {
-  T v[kBV];
-};
-
-template <typename T>
-__device__ __forceinline__ RowV<T> ldv(const T *p) {
-  typedef typename VecB<T>::type VT;
-  const VT x = __ldg(reinterpret_cast<const VT *>(p));
-  RowV<T> r;
-  memcpy(r.v, &x, sizeof(VT));
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ RowV<T> ldv_rw(const T *p) {
-  typedef typename VecB<T>::type VT;
-  const VT x = *reinterpret_cast<const VT *>(p);
-  RowV<T> r;
-  memcpy(r.v, &x, sizeof(VT));
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ void stv(T *p, const RowV<T> &r) {
-  typedef typename VecB<T>::type VT;
-  VT x;
-  memcpy(&x, r.v, sizeof(VT));
-  *reinterpret_cast<VT *>(p) = x;
-}
-
-// The vector accesses at element i of an array of n elements, checked like
-// ldg_c / ld_c / st_c (both elements must lie inside).
-template <typename T>
-__device__ __forceinline__ RowV<T> ldv_c(const T *a, long long i, long long n, int *status) {
-  if (in_bounds(i + kBV - 1, n, status) && in_bounds(i, n, status)) return ldv(a + i);
-  RowV<T> r;
-#pragma unroll
-  for (int c = 0; c < kBV; ++c) r.v[c] = T(0);
-  return r;
-}
-template <typename T>
-__device__ __forceinline__ RowV<T> ldv_rw_c(const T *a, long long i, long long n, int *status) {
-  if (in_bounds(i + kBV - 1, n, status) && in_bounds(i, n, status)) return ldv_rw(a + i);
-  RowV<T> r;
-#pragma unroll
-  for (int c = 0; c < kBV; ++c) r.v[c] = T(0);
-  return r;
-}
-template <typename T>
-__device__ __forceinline__ void stv_c(T *a, long long i, long long n, int *status, const RowV<T> &r) {
-  if (in_bounds(i + kBV - 1, n, status) && in_bounds(i, n, status)) stv(a + i, r);
-}
-
-// psi_H of the face in slot F at one cell (cpml_border.cpp:499-527): updates
-// the layer arrays and adds the face's currents to m (MPulse's order: slots
-// in turn, as b_cell sums them).  d0 / d1: the differences of E along the
-// face's axis for psi0 / psi1.
-template <typename T, int F>
-__device__ __forceinline__ void b_face(const BParams<T> &p, int i, int j, int k, T d0, T d1, T (&m)[3]) {
-  constexpr int dim = face_axis(F);
-  const CpmlFace<T> &L = p.cpml[F];
-  const int idx = dim == 0 ? i + 1 : dim == 1 ? j + 1 : k;
-  int li;
-  if (dim == 2) li = ((k - L.lo) * p.ny + j) * p.nx + i;
-  else if (dim == 0) li = ((k - L.zlo) * p.ny + j) * L.ex + (i + 1 - L.lo);
-  else li = ((k - L.zlo) * L.ey + (j + 1 - L.lo)) * p.nx + i;
-  const T b = ld(L.b + idx), c = ld(L.c + idx);
-  const T c0 = b * ld_c(L.psi0, li, L.n, p.status) + c * d0;
-  const T c1 = b * ld_c(L.psi1, li, L.n, p.status) + c * d1;
-  st_c(L.psi0, li, L.n, p.status, c0);
-  st_c(L.psi1, li, L.n, p.status, c1);
-  if (dim == 2) { m[0] += c0; m[1] += c1; }
-  else if (dim == 0) { m[1] += c0; m[2] += c1; }
-  else { m[2] += c0; m[0] += c1; }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(32 * MPB_B_BLOCK_Y,
-                                  (sizeof(T) == 4 ? MPB_BV_MIN_THREADS_F : MPB_BV_MIN_THREADS_D) / (32 * MPB_B_BLOCK_Y))
-    b_half_vec_kernel(const BParams<T> p) {
-  constexpr int V = kBV;
-  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i0 >= p.nx || j >= p.ny) return;
-  const int k0 = p.k_first + blockIdx.z * p.kchunk;
-  const int k1 = min(k0 + p.kchunk - 1, p.k_last);
-  if (k0 > k1) return;
-
-  const long long plane = p.plane;
-  const int jp = (j == p.ny - 1) ? 0 : j + 1;
-  const int il = (i0 + V == p.nx) ? 0 : i0 + V;  // x+1 of the last cell
-  const long long col = (long long)j * p.nx + i0;
-  const long long colyp = (long long)jp * p.nx + i0;
-  const long long colxl = (long long)j * p.nx + il;
-  const T *__restrict__ Ex = p.E[0];
-  const T *__restrict__ Ey = p.E[1];
-  const T *__restrict__ Ez = p.E[2];
-  T *__restrict__ Bx = p.B[0];
-  T *__restrict__ By = p.B[1];
-  T *__restrict__ Bz = p.B[2];
-  T ikx[V];
-#pragma unroll
-  for (int c = 0; c < V; ++c) ikx[c] = ld(p.ik[0] + i0 + c + 1);
-  const T iky = ld(p.ik[1] + j + 1);
-  const T iky_bz = ld(p.ik_bz_y + j + 1);
-  // y faces (slots 0, 1) hold whole rows: warp-uniform; x faces (slots 2, 3)
-  // per cell, bits 2c and 2c + 1
-  const unsigned ybits = face_column_mask(p.cpml, i0, j) & 3u;
-  unsigned xbits = 0;
-#pragma unroll
-  for (int c = 0; c < V; ++c) xbits |= ((face_column_mask(p.cpml, i0 + c, j) >> 2) & 3u) << (2 * c);
-  const int2 srck = source_plane_range(p);
-
-  const long long nf = p.n_field;
-  int *const st = p.status;
-  RowV<T> ex = ldv_c(Ex, (long long)k0 * plane + col, nf, st), ey = ldv_c(Ey, (long long)k0 * plane + col, nf, st);
-  for (int k = k0; k <= k1; ++k) {
-    const long long base = (long long)k * plane;
-    int kp = k + 1;
-    if (p.zperiodic && kp == p.nz + 1) kp = 1;
-    const long long basep = (long long)kp * plane;
+    const long long basep = (p.zperiodic && k == p.nz ? 1 : k + 1) * plane;
     // ---- every load of this plane first
-    const RowV<T> ex_kp = ldv_c(Ex, basep + col, nf, st), ey_kp = ldv_c(Ey, basep + col, nf, st);
-    const RowV<T> ez = ldv_c(Ez, base + col, nf, st);
-    const T ez_xl = ldg_c(Ez, base + colxl, nf, st), ey_xl = ldg_c(Ey, base + colxl, nf, st);
-    const RowV<T> ez_yp = ldv_c(Ez, base + colyp, nf, st), ex_yp = ldv_c(Ex, base + colyp, nf, st);
-    const RowV<T> bx = ldv_rw_c(Bx, base + col, nf, st), by = ldv_rw_c(By, base + col, nf, st),
-                  bz = ldv_rw_c(Bz, base + col, nf, st);
+    const RowV<T, V> ex_kp = ldp<V>(Ex, basep, col, nf, st), ey_kp = ldp<V>(Ey, basep, col, nf, st);
+    const RowV<T, V> ez = ldp<V>(Ez, base, col, nf, st);
+    const RowV<T, V> bx = ldp<V>(Bx, base, col, nf, st), by = ldp<V>(By, base, col, nf, st),
+                     bz = ldp<V>(Bz, base, col, nf, st);
+    const RowV<T, V> ez_yp = ldp<V>(Ez, base, colyp, nf, st), ex_yp = ldp<V>(Ex, base, colyp, nf, st);
+    const RowV<T, 1> ez_xl = ldp<1>(Ez, base, colxp, nf, st), ey_xl = ldp<1>(Ey, base, colxp, nf, st);
     const T ikz = ld(p.ik[2] + k);
-    // ---- H-side currents, in MPulse's order: faces by slot, then the injector
-    T m[V][3];
-#pragma unroll
-    for (int c = 0; c < V; ++c) m[c][0] = m[c][1] = m[c][2] = T(0);
-    if (ybits) {
-#pragma unroll
-      for (int c = 0; c < V; ++c) {
-        const T d0 = ex_yp.v[c] - ex.v[c], d1 = -(ez_yp.v[c] - ez.v[c]);
-        if (ybits & 1u) b_face<T, 0>(p, i0 + c, j, k, d0, d1, m[c]);
-        if (ybits & 2u) b_face<T, 1>(p, i0 + c, j, k, d0, d1, m[c]);
-      }
+    if (g.ahead && k < k1) {
+      const long long ba = base + plane;
+      prefetch_l2(Bx + ba + col);
+      prefetch_l2(By + ba + col);
+      prefetch_l2(Bz + ba + col);
+      prefetch_l2(Ex + ba + plane + col);
+      prefetch_l2(Ey + ba + plane + col);
+      prefetch_l2(Ez + ba + col);
     }
-    if (xbits) {
-#pragma unroll
-      for (int c = 0; c < V; ++c) {
-        const T ezx = c + 1 < V ? ez.v[c + 1 < V ? c + 1 : 0] : ez_xl;
-        const T eyx = c + 1 < V ? ey.v[c + 1 < V ? c + 1 : 0] : ey_xl;
-        const T d0 = ezx - ez.v[c], d1 = -(eyx - ey.v[c]);
-        if (xbits & (1u << (2 * c))) b_face<T, 2>(p, i0 + c, j, k, d0, d1, m[c]);
-        if (xbits & (2u << (2 * c))) b_face<T, 3>(p, i0 + c, j, k, d0, d1, m[c]);
-      }
-    }
-    if (z_face_plane(p.cpml, k)) {
-      const bool z4 = p.cpml[4].active && k >= p.cpml[4].lo && k <= p.cpml[4].hi;
-      const bool z5 = p.cpml[5].active && k >= p.cpml[5].lo && k <= p.cpml[5].hi;
-#pragma unroll
-      for (int c = 0; c < V; ++c) {
-        const T d0 = ey_kp.v[c] - ey.v[c], d1 = -(ex_kp.v[c] - ex.v[c]);
-        if (z4) b_face<T, 4>(p, i0 + c, j, k, d0, d1, m[c]);
-        if (z5) b_face<T, 5>(p, i0 + c, j, k, d0, d1, m[c]);
-      }
-    }
-    if (k >= srck.x && k <= srck.y) {
-      for (int s = 0; s < p.n_src; ++s) {
-        if (k != p.src[s].plane) continue;
-#pragma unroll
-        for (int c = 0; c < V; ++c) {
-          const T sa = ldg_c(p.src[s].v0, col + c, p.plane, st), sb = ldg_c(p.src[s].v1, col + c, p.plane, st);
-          for (int q = 0; q < p.src_mult; ++q) {
-            m[c][0] += sa;
-            m[c][1] += sb;
-          }
-        }
-      }
-    }
-    // ---- plrcStepB (fdtd_plrc.cpp:263-293)
-    const T dt = p.dt;
-    RowV<T> bxn, byn, bzn;
+
+    // ---- the differences of E, then the H-side currents in MPulse's order
+    T dzy[V], dyz[V], dxz[V], dzx[V], dyx[V], dxy[V];  // d<component><axis>
 #pragma unroll
     for (int c = 0; c < V; ++c) {
-      const T ezx = c + 1 < V ? ez.v[c + 1 < V ? c + 1 : 0] : ez_xl;
-      const T eyx = c + 1 < V ? ey.v[c + 1 < V ? c + 1 : 0] : ey_xl;
-      // (the sums of two products are left to the compiler here: spelled out
-      // as in b_cell they cost this kernel six registers and 7% of its time;
-      // the results agree with b_cell's to the last bit or within rounding)
-      bxn.v[c] = bx.v[c] + dt_mul(dt, p.dt_lo, (ey_kp.v[c] - ey.v[c]) * ikz - (ez_yp.v[c] - ez.v[c]) * iky + m[c][0]);
-      byn.v[c] = by.v[c] + dt_mul(dt, p.dt_lo, (ezx - ez.v[c]) * ikx[c] - (ex_kp.v[c] - ex.v[c]) * ikz + m[c][1]);
-      bzn.v[c] = bz.v[c] + dt_mul(dt, p.dt_lo, (ex_yp.v[c] - ex.v[c]) * iky_bz - (eyx - ey.v[c]) * ikx[c] + m[c][2]);
+      dzy[c] = ez_yp.v[c] - ez.v[c];
+      dxy[c] = ex_yp.v[c] - ex.v[c];
+      dzx[c] = (c + 1 < V ? ez.v[c + 1 < V ? c + 1 : 0] : ez_xl.v[0]) - ez.v[c];
+      dyx[c] = (c + 1 < V ? ey.v[c + 1 < V ? c + 1 : 0] : ey_xl.v[0]) - ey.v[c];
+      dxz[c] = ex_kp.v[c] - ex.v[c];
+      dyz[c] = ey_kp.v[c] - ey.v[c];
     }
-    stv_c(Bx, base + col, nf, st, bxn);
-    stv_c(By, base + col, nf, st, byn);
-    stv_c(Bz, base + col, nf, st, bzn);
+    T cur[V][3];
+#pragma unroll
+    for (int c = 0; c < V; ++c) cur[c][0] = cur[c][1] = cur[c][2] = T(0);
+    const bool zlow = k <= g.lo[2], zhigh = k >= g.hi[2];
+    if (fmask || zlow || zhigh) {
+      T nzy[V], nyx[V], nxz[V];
+#pragma unroll
+      for (int c = 0; c < V; ++c) {
+        nzy[c] = -dzy[c];
+        nyx[c] = -dyx[c];
+        nxz[c] = -dxz[c];
+      }
+      face_currents<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, dxy, nzy, dzx, nyx, dyz, nxz, cur, st);
+    }
+    if (k == g.src) source_currents<T, V>(p, col, cur);
+
+    // ---- plrcStepB (fdtd_plrc.cpp:263-293)
+    RowV<T, V> bxn, byn, bzn;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      bxn.v[c] = add_dt(bx.v[c], p.dt, p.dt_lo, fma_pm(dyz[c], ikz, dzy[c], iky) + cur[c][0]);
+      byn.v[c] = add_dt(by.v[c], p.dt, p.dt_lo, fma_pm(dzx[c], ikx.v[c], dxz[c], ikz) + cur[c][1]);
+      bzn.v[c] = add_dt(bz.v[c], p.dt, p.dt_lo, fma_pm(dxy[c], iky_bz, dyx[c], ikx.v[c]) + cur[c][2]);
+    }
+    stp<V>(Bx, base, col, nf, st, bxn);
+    stp<V>(By, base, col, nf, st, byn);
+    stp<V>(Bz, base, col, nf, st, bzn);
     ex = ex_kp;
     ey = ey_kp;
   }
@@ -523,24 +495,89 @@ __global__ void __launch_bounds__(32 * MPB_B_BLOCK_Y,
 // ---------------------------------------------------------------------------
 // Launchers (called from mp_api.cu)
 
-
-template <typename T, int MODE, bool DESIGN, bool PLASMA = false>
-static cudaError_t launch_e_np(const EParams<T> &p, int np, cudaStream_t st) {
-  const int nk = p.k_last - p.k_first + 1;
-  const long long bxy = (long long)((p.nx + 31) / 32) * ((p.ny + MPB_E_BLOCK_Y - 1) / MPB_E_BLOCK_Y);
-  const long long per_sm = sizeof(T) == 4 ? MPB_E_BLOCKS_PER_SM_F : MPB_E_BLOCKS_PER_SM_D;
-  const long long chunks = std::max(1LL, (148LL * per_sm + bxy - 1) / bxy);
-  EParams<T> q = p;
-  q.kchunk = int(std::min<long long>(nk, std::max<long long>(MPB_E_MIN_PLANES, (nk + chunks - 1) / chunks)));
-  const dim3 g((p.nx + 31) / 32, (p.ny + MPB_E_BLOCK_Y - 1) / MPB_E_BLOCK_Y, (nk + q.kchunk - 1) / q.kchunk),
-      b(32, MPB_E_BLOCK_Y, 1);
-  switch (np) {
-    case 0: e_half_kernel<T, MODE, 0, DESIGN, PLASMA><<<g, b, 0, st>>>(q); break;
-    case 1: e_half_kernel<T, MODE, 1, DESIGN, PLASMA><<<g, b, 0, st>>>(q); break;
-    case 2: e_half_kernel<T, MODE, 2, DESIGN, PLASMA><<<g, b, 0, st>>>(q); break;
-    default: e_half_kernel<T, MODE, 3, DESIGN, PLASMA><<<g, b, 0, st>>>(q); break;
+// The grid of a half step: V cells per thread, z-chunks of the planes.
+// Planes per block: one where two would leave SMs without four blocks (32^3
+// FP64: E 9.1 instead of 10.2 us); else at least two, and more while 50 blocks
+// per SM remain, up to max_planes.  Longer chunks save the two carried loads of
+// each chunk's first plane but leave fewer warps and a longer tail (256 x 256 x
+// 512 FP32 E half with 2 / 4 / 8 / 16 / 24 planes 725 / 682 / 677 / 700 / 715 us,
+// 128 x 128 x 256 112 / 107 / 112 us with 2 / 4 / 8).  The prefetch is for
+// states that do not stay in L2 (126 MB): 256 x 256 x 512 E half 748 -> 677 us,
+// 120 x 104 x 136 FP64 93 -> 89; on a 99 MB state 29.8 -> 31.5.
+template <typename P>
+static RowGrid row_grid(const P &p, int V, int max_planes, dim3 *d) {
+  RowGrid r;
+  r.nrow = unsigned(p.nx / V);
+  r.nvec = r.nrow * unsigned((p.ny + kRowTile - 1) / kRowTile);
+  // nrow >= 2; exact for every t < 2^31 with shift = ceil(log2(nrow)) - 1 and
+  // mul = ceil(2^(32 + shift) / nrow) (Granlund and Montgomery, PLDI 1994)
+  int l = 0;
+  while ((1ULL << l) < r.nrow) ++l;
+  r.shift = unsigned(l - 1);
+  r.mul = unsigned(((1ULL << (32 + r.shift)) + r.nrow - 1) / r.nrow);
+  const int axis_high[3] = {2, 0, 4};  // the slot of the high face; the low one follows
+  for (int a = 0; a < 3; ++a) {
+    const auto &H = p.cpml[axis_high[a]], &L = p.cpml[axis_high[a] + 1];
+    r.hi[a] = H.active ? H.lo : 1 << 30;
+    r.lo[a] = L.active ? L.hi : -1;
   }
-  return cudaGetLastError();
+  r.src = p.n_src > 0 ? p.src[0].plane : -1;
+  const int nk = p.k_last - p.k_first + 1;
+  const long long bxy = (r.nvec + 31) / 32, all = bxy * nk;
+  r.kchunk = all < 2 * 148 * 4 ? 1 : int(std::min<long long>(std::max(2LL, all / (148 * 50)), max_planes));
+  r.kchunk = std::max(r.kchunk, (nk + 65534) / 65535);  // blocks in y
+  r.ahead = p.state_bytes > (160LL << 20);
+  *d = dim3(unsigned(bxy), unsigned((nk + r.kchunk - 1) / r.kchunk), 1);
+  return r;
+}
+
+// A launch that lets the kernel's blocks start before the previous kernel of
+// the stream has finished (programmatic dependent launch): they set up their
+// columns and faces and wait (griddepcontrol.wait) before the first load of the
+// state.  32^3 FP64: 6.0 -> 5.2 us per step, 64^3 FP32 9.1 -> 8.7.
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_row(void (*kernel)(KArgs...), dim3 g, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = g;
+  cfg.blockDim = dim3(kRowThreads, 1, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename T>
+constexpr int max_planes() {
+  return sizeof(T) == 4 ? 8 : 4;
+}
+
+template <typename T, int V, int MODE, bool DESIGN, bool PLASMA>
+static cudaError_t launch_e_v(const EParams<T> &p, int np, cudaStream_t st) {
+  constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
+  dim3 d;
+  const RowGrid g = row_grid(p, V, max_planes<T>(), &d);
+  switch (PLRC ? np : 0) {
+    case 0: return launch_row(e_half_kernel<T, V, MODE, 0, DESIGN, PLASMA>, d, st, p, g);
+    case 1: return launch_row(e_half_kernel<T, V, MODE, PLRC ? 1 : 0, DESIGN, PLASMA>, d, st, p, g);
+    case 2: return launch_row(e_half_kernel<T, V, MODE, PLRC ? 2 : 0, DESIGN, PLASMA>, d, st, p, g);
+    default: return launch_row(e_half_kernel<T, V, MODE, PLRC ? 3 : 0, DESIGN, PLASMA>, d, st, p, g);
+  }
+}
+
+// Two cells per thread in FP32 where the update is short (150 x 131 x 210
+// fdtd-plain 30 instead of 38 us, 160 x 144 x 250 PLRC with one pole 79 instead
+// of 81, 128^3 with two poles 46 instead of 49); one with Kerr or the plasma
+// plug-ins (128 x 128 x 256 Kerr 108 instead of 113 us, 128 x 128 x 192 plasma
+// 109 instead of 116), with a design region (96^3 21.6 instead of 23.0) and in
+// FP64, whose two-cell form spills (192 x 192 x 384 551 instead of 691 us).
+template <typename T, int MODE, bool DESIGN, bool PLASMA>
+static cudaError_t launch_e_np(const EParams<T> &p, int np, cudaStream_t st) {
+  constexpr int V = sizeof(T) == 4 && MODE != MODE_PLRC_NONLIN && !DESIGN && !PLASMA ? 2 : 1;
+  return p.nx % V == 0 && p.nx > V ? launch_e_v<T, V, MODE, DESIGN, PLASMA>(p, np, st)
+                                   : launch_e_v<T, 1, MODE, DESIGN, PLASMA>(p, np, st);
 }
 
 template <typename T>
@@ -550,43 +587,32 @@ cudaError_t launch_e_half(const EParams<T> &p, int mode, int np, cudaStream_t st
   const bool design = p.design.x0 <= p.design.x1;
   const bool plasma = p.rho != nullptr;
   switch (mode) {
-    case MODE_PLAIN: return launch_e_np<T, MODE_PLAIN, false>(p, 0, st);
-    case MODE_NL: return launch_e_np<T, MODE_NL, false>(p, 0, st);
+    case MODE_PLAIN: return launch_e_np<T, MODE_PLAIN, false, false>(p, 0, st);
+    case MODE_NL: return launch_e_np<T, MODE_NL, false, false>(p, 0, st);
     case MODE_PLRC_LIN:
-      return design   ? launch_e_np<T, MODE_PLRC_LIN, true>(p, np, st)
+      return design   ? launch_e_np<T, MODE_PLRC_LIN, true, false>(p, np, st)
              : plasma ? launch_e_np<T, MODE_PLRC_LIN, false, true>(p, np, st)
-                      : launch_e_np<T, MODE_PLRC_LIN, false>(p, np, st);
+                      : launch_e_np<T, MODE_PLRC_LIN, false, false>(p, np, st);
     default:
-      return design   ? launch_e_np<T, MODE_PLRC_NONLIN, true>(p, np, st)
+      return design   ? launch_e_np<T, MODE_PLRC_NONLIN, true, false>(p, np, st)
              : plasma ? launch_e_np<T, MODE_PLRC_NONLIN, false, true>(p, np, st)
-                      : launch_e_np<T, MODE_PLRC_NONLIN, false>(p, np, st);
+                      : launch_e_np<T, MODE_PLRC_NONLIN, false, false>(p, np, st);
   }
 }
 
+template <typename T, int V>
+static cudaError_t launch_b_v(const BParams<T> &p, cudaStream_t st) {
+  dim3 d;
+  const RowGrid g = row_grid(p, V, max_planes<T>(), &d);
+  return launch_row(b_half_kernel<T, V>, d, st, p, g);
+}
+
+// Two cells per thread in FP32 (256 x 256 x 512: 257 us, one cell 293, four
+// 338), one in FP64 (192 x 192 x 384: 198 us, two cells 217).
 template <typename T>
 cudaError_t launch_b_half(const BParams<T> &p, cudaStream_t st) {
-  const int nk = p.k_last - p.k_first + 1;
-#if MPB_B_VECTOR
-  constexpr int V = kBV;
-  // rows of whole warps only: on narrow grids (nx = 96: 48 threads a row)
-  // the scalar kernel keeps every lane busy
-  if (p.nx % (32 * V) == 0) {
-    // V cells per thread: z-chunks sized for a number of blocks per SM, at
-    // least 8 planes each
-    const int tx = p.nx / V;
-    const long long per_sm = sizeof(T) == 4 ? MPB_BV_BLOCKS_PER_SM_F : MPB_BV_BLOCKS_PER_SM_D;
-    const long long bxy = (long long)(tx / 32) * ((p.ny + MPB_B_BLOCK_Y - 1) / MPB_B_BLOCK_Y);
-    const long long chunks = std::max(1LL, (148LL * per_sm + bxy - 1) / bxy);
-    BParams<T> q = p;
-    q.kchunk = int(std::max<long long>(MPB_BV_MIN_PLANES, (nk + chunks - 1) / chunks));
-    const dim3 g((tx + 31) / 32, (p.ny + MPB_B_BLOCK_Y - 1) / MPB_B_BLOCK_Y, (nk + q.kchunk - 1) / q.kchunk);
-    b_half_vec_kernel<T><<<g, dim3(32, MPB_B_BLOCK_Y, 1), 0, st>>>(q);
-    return cudaGetLastError();
-  }
-#endif
-  const dim3 g((p.nx + 31) / 32, (p.ny + MPB_B_BLOCK_Y - 1) / MPB_B_BLOCK_Y, (nk + p.kchunk - 1) / p.kchunk);
-  b_half_kernel<T><<<g, dim3(32, MPB_B_BLOCK_Y, 1), 0, st>>>(p);
-  return cudaGetLastError();
+  constexpr int V = sizeof(T) == 4 ? 2 : 1;
+  return p.nx % V == 0 && p.nx > V ? launch_b_v<T, V>(p, st) : launch_b_v<T, 1>(p, st);
 }
 
 template cudaError_t launch_e_half<float>(const EParams<float> &, int, int, cudaStream_t);
