@@ -34,6 +34,7 @@
 // thread per (x, y) column and chunk of planes.
 #include "mp_checked.cuh"
 #include "mp_device.h"
+#include "mp_pdl.cuh"
 
 #include <cuda_runtime.h>
 
@@ -102,12 +103,6 @@ __device__ __forceinline__ void face_w(const AdjFace<T> &F, int pos, int li, R c
     w0 = w1 = R(0);
   }
 }
-
-// Programmatic dependent launch: let the next kernel of the stream start its
-// blocks, and wait until the previous kernel's writes are visible.  Both are
-// no-ops for a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 }  // namespace
 
@@ -681,36 +676,43 @@ __global__ void __launch_bounds__(256) adj_init_kernel(const AdjParams<T> p) {
   }
 }
 
-// One step's objective term into out[slot]: one block, FP64, fixed order.
+// One step's objective term as gridDim.x partial sums, out[block], FP64 in a
+// fixed order.  `lanes` threads (a power of two) run along a row of the box, so
+// a block takes 256 / lanes rows at a time.  Latency-bound at the sizes in use:
+// with the one block of 256 threads that it had, the term of a 128 x 128 plane
+// cost 37 us a step beside 162 us of half steps, that of an 8^3 box 4.6; with
+// four cells per thread 5 and 2.5 (launched early, beside the half steps).
 template <typename T>
 __global__ void __launch_bounds__(256) objective_term_kernel(const T *Ex, const T *Ey, const T *Ez, const T *Bx,
-                                                             const T *By, int nx, int ny, long long plane, int kind,
-                                                             int x0, int x1, int y0, int y1, int z0, int z1,
-                                                             double f, double *out) {
-  __shared__ double red[256];
-  const int bx = x1 - x0 + 1, by = y1 - y0 + 1, bz = z1 - z0 + 1;
-  const long long n = (long long)bx * by * bz;
+                                                             const T *By, int nx, long long plane, int kind, int x0,
+                                                             int x1, int y0, unsigned by, int z0, unsigned rows,
+                                                             int lanes, double f, double *out) {
+  __shared__ double red[8];
+  pdl_launch_dependents();
+  const unsigned per = 256u / unsigned(lanes);
+  const int lane = threadIdx.x & (lanes - 1);
   double acc = 0.0;
-  for (long long q = threadIdx.x; q < n; q += blockDim.x) {
-    const int i = x0 + int(q % bx);
-    const long long r = q / bx;
-    const int j = y0 + int(r % by);
-    const int k = z0 + int(r / by);
-    const long long c = (long long)k * plane + (long long)j * nx + i;
-    if (kind == 1) {
-      const double ex = Ex[c], ey = Ey[c], ez = Ez[c];
-      acc += ex * ex + ey * ey + ez * ez;
-    } else {
-      acc += (double)Ex[c] * (double)By[c] - (double)Ey[c] * (double)Bx[c];
+  pdl_wait();
+  for (unsigned r = blockIdx.x * per + threadIdx.x / unsigned(lanes); r < rows; r += gridDim.x * per) {
+    const unsigned k = r / by;
+    const long long row = (long long)(z0 + int(k)) * plane + (long long)(y0 + int(r - k * by)) * nx;
+    for (int i = x0 + lane; i <= x1; i += lanes) {
+      const long long c = row + i;
+      if (kind == 1) {
+        const double ex = Ex[c], ey = Ey[c], ez = Ez[c];
+        acc += ex * ex + ey * ey + ez * ez;
+      } else {
+        acc += (double)Ex[c] * (double)By[c] - (double)Ey[c] * (double)Bx[c];
+      }
     }
   }
-  red[threadIdx.x] = acc;
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) acc += red[w];
+    out[blockIdx.x] = f * acc;
   }
-  if (threadIdx.x == 0) *out = f * red[0];
 }
 
 __global__ void __launch_bounds__(256) sum_terms_kernel(const double *terms, long long n, double *out) {
@@ -728,24 +730,6 @@ __global__ void __launch_bounds__(256) sum_terms_kernel(const double *terms, lon
 
 // ---------------------------------------------------------------------------
 // Launchers
-
-// A launch with programmatic stream serialisation (the kernel's blocks may
-// start before the previous kernel in the stream has finished; the kernel
-// orders its reads with griddepcontrol.wait).
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 g, dim3 b, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = g;
-  cfg.blockDim = b;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 
 template <typename T>
 cudaError_t launch_adj_e(const AdjParams<T> &p, cudaStream_t st) {
@@ -787,12 +771,22 @@ cudaError_t launch_adj_init(const AdjParams<T> &p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Blocks (partial sums) of a step's term over a box: four cells per thread, at
+// most one block per SM.
+int objective_blocks(const int box0[6]) {
+  const long long cells =
+      (long long)(box0[1] - box0[0] + 1) * (box0[3] - box0[2] + 1) * (box0[5] - box0[4] + 1);
+  return int(cells > 1024 * 148 ? 148 : (cells + 1023) / 1024);
+}
+
 template <typename T>
-cudaError_t launch_objective_term(const T *const E[3], const T *const B[3], int nx, int ny, long long plane, int kind,
+cudaError_t launch_objective_term(const T *const E[3], const T *const B[3], int nx, long long plane, int kind,
                                   const int box0[6], double f, double *out, cudaStream_t st) {
-  objective_term_kernel<T><<<1, 256, 0, st>>>(E[0], E[1], E[2], B[0], B[1], nx, ny, plane, kind, box0[0], box0[1],
-                                              box0[2], box0[3], box0[4], box0[5], f, out);
-  return cudaGetLastError();
+  const unsigned by = unsigned(box0[3] - box0[2] + 1), rows = by * unsigned(box0[5] - box0[4] + 1);
+  int lanes = 1;
+  while (lanes < 32 && lanes < box0[1] - box0[0] + 1) lanes *= 2;
+  return launch_pdl(objective_term_kernel<T>, dim3(objective_blocks(box0), 1, 1), dim3(256, 1, 1), st, E[0], E[1],
+                    E[2], B[0], B[1], nx, plane, kind, box0[0], box0[1], box0[2], by, box0[4], rows, lanes, f, out);
 }
 
 cudaError_t launch_sum_terms(const double *terms, long long n, double *out, cudaStream_t st) {
@@ -806,9 +800,9 @@ template cudaError_t launch_adj_b<float>(const AdjParams<float> &, cudaStream_t)
 template cudaError_t launch_adj_b<double>(const AdjParams<double> &, cudaStream_t);
 template cudaError_t launch_adj_init<float>(const AdjParams<float> &, cudaStream_t);
 template cudaError_t launch_adj_init<double>(const AdjParams<double> &, cudaStream_t);
-template cudaError_t launch_objective_term<float>(const float *const[3], const float *const[3], int, int, long long,
-                                                  int, const int[6], double, double *, cudaStream_t);
-template cudaError_t launch_objective_term<double>(const double *const[3], const double *const[3], int, int,
-                                                   long long, int, const int[6], double, double *, cudaStream_t);
+template cudaError_t launch_objective_term<float>(const float *const[3], const float *const[3], int, long long, int,
+                                                  const int[6], double, double *, cudaStream_t);
+template cudaError_t launch_objective_term<double>(const double *const[3], const double *const[3], int, long long, int,
+                                                   const int[6], double, double *, cudaStream_t);
 
 }  // namespace mpb

@@ -61,9 +61,10 @@ template <typename T> cudaError_t launch_adj_e(const AdjParams<T> &, cudaStream_
 template <typename T> cudaError_t launch_adj_b(const AdjParams<T> &, cudaStream_t);
 template <typename T> cudaError_t launch_adj_init(const AdjParams<T> &, cudaStream_t);
 template <typename T>
-cudaError_t launch_objective_term(const T *const E[3], const T *const B[3], int nx, int ny, long long plane, int kind,
+cudaError_t launch_objective_term(const T *const E[3], const T *const B[3], int nx, long long plane, int kind,
                                   const int box0[6], double f, double *out, cudaStream_t st);
 cudaError_t launch_sum_terms(const double *terms, long long n, double *out, cudaStream_t st);
+int objective_blocks(const int box0[6]);
 }  // namespace mpb
 
 using namespace mpb;
@@ -1648,21 +1649,31 @@ void objective_box(const mp_adjoint_config *a, int b0[6]) {
   b0[5] = a->kind == MP_OBJ_E2_BOX ? a->box[5] : a->box[4];
 }
 
+// The partial sums a step's objective term is written as.
+int objective_parts(const mp_adjoint_config *a) {
+  int b0[6];
+  objective_box(a, b0);
+  return objective_blocks(b0);
+}
+
+// The objective term of the live state into the partial sums of step n.
 template <typename T>
-int objective_term(mp_ctx *c, const mp_adjoint_config *a, double *out) {
+int objective_term(mp_ctx *c, const mp_adjoint_config *a, double *terms, long long n) {
   const mp_config &g = c->cfg;
   const T *E[3] = {static_cast<const T *>(c->F[0]), static_cast<const T *>(c->F[1]), static_cast<const T *>(c->F[2])};
   const T *B[3] = {static_cast<const T *>(c->F[3]), static_cast<const T *>(c->F[4]), static_cast<const T *>(c->F[5])};
   int b0[6];
   objective_box(a, b0);
   const double f = a->kind == MP_OBJ_E2_BOX ? g.dt : g.dt * g.dx * g.dy;
-  cudaError_t e = launch_objective_term<T>(E, B, g.nx, g.ny, c->plane, a->kind, b0, f, out, c->stream);
+  cudaError_t e = launch_objective_term<T>(E, B, g.nx, c->plane, a->kind, b0, f, terms + n * objective_blocks(b0), c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "objective kernel");
   c->launches++;
   return MP_OK;
 }
 
-int read_sum(mp_ctx *c, double *terms, long long n, double *J) {
+// J: the sum of the partial sums of all steps (the result goes after them).
+int read_sum(mp_ctx *c, const mp_adjoint_config *a, double *terms, double *J) {
+  const long long n = (long long)a->steps * objective_parts(a);
   cudaError_t e = launch_sum_terms(terms, n, terms + n, c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "sum kernel");
   c->launches++;
@@ -1677,13 +1688,13 @@ template <typename T>
 int objective_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_config *a, double *J) {
   DevBufs buf(c->stream);
   double *terms;
-  cudaError_t e = buf.alloc(reinterpret_cast<void **>(&terms), (size_t(a->steps) + 1) * sizeof(double));
+  cudaError_t e = buf.alloc(reinterpret_cast<void **>(&terms), (size_t(a->steps) * objective_parts(a) + 1) * sizeof(double));
   if (e != cudaSuccess) return cuda_err(c, e, "objective allocation");
   StepHooks h;
-  h.after = [&](long long n) { return objective_term<T>(c, a, terms + n); };
+  h.after = [&](long long n) { return objective_term<T>(c, a, terms, n); };
   int rc = step_impl<T>(c, ep, bp, a->steps, nullptr, nullptr, &h);
   if (rc != MP_OK) return rc;
-  rc = read_sum(c, terms, a->steps, J);
+  rc = read_sum(c, a, terms, J);
   return rc != MP_OK ? rc : mp_check_status(c);
 }
 
@@ -1948,7 +1959,7 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
   } else {
     if ((e = sbuf.alloc(reinterpret_cast<void **>(&ckpt), size_t(slots + 1) * S)) != cudaSuccess ||
         (e = sbuf.alloc(reinterpret_cast<void **>(&hist[0]), size_t(K + 1) * H)) != cudaSuccess ||
-        (e = sbuf.alloc(reinterpret_cast<void **>(&terms), (size_t(Tn) + 1) * sizeof(double))) != cudaSuccess)
+        (e = sbuf.alloc(reinterpret_cast<void **>(&terms), (size_t(Tn) * objective_parts(a) + 1) * sizeof(double))) != cudaSuccess)
       return cuda_err(c, e, "checkpoint allocation");
     if (nbuf == 2 && sbuf.alloc(reinterpret_cast<void **>(&hist[1]), size_t(K + 1) * H) != cudaSuccess) {
       cudaGetLastError();  // no room for the second buffer: chunks run forward and back in turn
@@ -2133,7 +2144,7 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
   // Forward steps n0..n1-1 from the live state in one batched call: the E
   // kernel of step n stores the new E into history slot n + 1 - h0 when
   // n >= h0 (h0 < 0: no history), the Sz planes are copied after it, and the
-  // objective term of every step not run before goes to terms[n].
+  // objective term of every step not run before goes to the terms of step n.
   auto run = [&](long long n0, long long n1, long long h0) -> int {
     StepHooks hk;
     hk.before = [&](long long q) {
@@ -2147,7 +2158,7 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
         const cudaError_t err = record(n + 1 - h0, false);
         if (err != cudaSuccess) return cuda_err(c, err, "history copy");
       }
-      return n >= reached ? objective_term<T>(c, a, terms + n) : MP_OK;
+      return n >= reached ? objective_term<T>(c, a, terms, n) : MP_OK;
     };
     const int r = step_impl<T>(c, ep, bp, int(n1 - n0), nullptr, nullptr, &hk);
     hist_into(-1);
@@ -2213,7 +2224,7 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
         // the first time the run reaches the end: J, the final state
         at_end = true;
         if ((err = copy_state(slots, true)) != cudaSuccess) return cuda_err(c, err, "checkpoint copy");
-        if ((r = read_sum(c, terms, Tn, J)) != MP_OK || (r = mp_check_status(c)) != MP_OK) return r;
+        if ((r = read_sum(c, a, terms, J)) != MP_OK || (r = mp_check_status(c)) != MP_OK) return r;
         if (phase == kAdjRecord) return kAdjStop;
       }
     }

@@ -38,6 +38,7 @@
 //   101 x 75 x 163 fdtd-nl FP64        E  49 ->  26   B  40 ->  17
 //   128 x 128 x 192 + plasma FP32      E 135 -> 109   B  56 ->  43
 #include "mp_cell.cuh"
+#include "mp_pdl.cuh"
 
 #include <algorithm>
 
@@ -71,13 +72,6 @@ namespace mpb {
 // rows 1% and 7% slower than 4.
 constexpr int kRowTile = 4;
 constexpr int kRowThreads = 32 * kRowTile;
-
-// Programmatic dependent launch: let the next kernel of the stream start its
-// blocks once all of this kernel's have started, and wait for the previous
-// kernel's writes.  Both are no-ops for a kernel launched without the attribute.
-// Every kernel of a chain waits, so the end of one is the end of all before it.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
@@ -531,24 +525,8 @@ static RowGrid row_grid(const P &p, int V, int max_planes, dim3 *d) {
   return r;
 }
 
-// A launch that lets the kernel's blocks start before the previous kernel of
-// the stream has finished (programmatic dependent launch): they set up their
-// columns and faces and wait (griddepcontrol.wait) before the first load of the
-// state.  32^3 FP64: 6.0 -> 5.2 us per step, 64^3 FP32 9.1 -> 8.7.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_row(void (*kernel)(KArgs...), dim3 g, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = g;
-  cfg.blockDim = dim3(kRowThreads, 1, 1);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
+// (Both kernels go out with programmatic dependent launch: 32^3 FP64 6.0 -> 5.2
+// us per step, 64^3 FP32 9.1 -> 8.7.)
 template <typename T>
 constexpr int max_planes() {
   return sizeof(T) == 4 ? 8 : 4;
@@ -560,10 +538,10 @@ static cudaError_t launch_e_v(const EParams<T> &p, int np, cudaStream_t st) {
   dim3 d;
   const RowGrid g = row_grid(p, V, max_planes<T>(), &d);
   switch (PLRC ? np : 0) {
-    case 0: return launch_row(e_half_kernel<T, V, MODE, 0, DESIGN, PLASMA>, d, st, p, g);
-    case 1: return launch_row(e_half_kernel<T, V, MODE, PLRC ? 1 : 0, DESIGN, PLASMA>, d, st, p, g);
-    case 2: return launch_row(e_half_kernel<T, V, MODE, PLRC ? 2 : 0, DESIGN, PLASMA>, d, st, p, g);
-    default: return launch_row(e_half_kernel<T, V, MODE, PLRC ? 3 : 0, DESIGN, PLASMA>, d, st, p, g);
+    case 0: return launch_pdl(e_half_kernel<T, V, MODE, 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
+    case 1: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 1 : 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
+    case 2: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 2 : 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
+    default: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 3 : 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
   }
 }
 
@@ -604,7 +582,7 @@ template <typename T, int V>
 static cudaError_t launch_b_v(const BParams<T> &p, cudaStream_t st) {
   dim3 d;
   const RowGrid g = row_grid(p, V, max_planes<T>(), &d);
-  return launch_row(b_half_kernel<T, V>, d, st, p, g);
+  return launch_pdl(b_half_kernel<T, V>, d, dim3(kRowThreads, 1, 1), st, p, g);
 }
 
 // Two cells per thread in FP32 (256 x 256 x 512: 257 us, one cell 293, four
