@@ -74,6 +74,7 @@ namespace {
 constexpr int kFaceOrderAll[6] = {FACE_NORTH, FACE_SOUTH, FACE_EAST, FACE_WEST, FACE_UP, FACE_DOWN};
 const int kFaceOrderZ[2] = {FACE_UP, FACE_DOWN};
 thread_local char g_create_err[512];
+constexpr size_t kTerms = 32768;  // doubles kept for mp_objective's terms
 constexpr size_t kKerrBytes = size_t(kKerrSlots) * kKerrStride * sizeof(unsigned long long);
 
 constexpr int face_dim(int f) {
@@ -92,6 +93,47 @@ struct LayerHost {
   size_t n = 0;
   void *psi0 = nullptr, *psi1 = nullptr;
   size_t b_off = 0, c_off = 0;  // offsets (elements) into the line buffer
+};
+
+// Device buffers laid out one after the other (256-byte aligned) in one
+// allocation: want() notes a buffer, commit() allocates for all noted since the
+// last commit, sets their pointers and, if asked, queues the zeroing of the whole
+// on the stream; free() (after the stream has drained) gives everything back.
+// One allocation, because a cudaMalloc / cudaFree pair of a few MB takes 0.6 ms
+// here (1 s at worst on a busy host): the 40 to 60 buffers of a context or of an
+// adjoint cost 24 ms, one buffer of the same size 2.
+struct Arena {
+  struct Want {
+    void **out;
+    size_t off;
+  };
+  std::vector<Want> wanted;
+  size_t need = 0;
+  std::vector<void *> blocks;
+  template <typename P>
+  void want(P **out, size_t bytes) {
+    *out = nullptr;
+    if (!bytes) return;
+    wanted.push_back({reinterpret_cast<void **>(out), need});
+    need += (bytes + 255) / 256 * 256;
+  }
+  cudaError_t commit(cudaStream_t st, bool zero) {
+    cudaError_t e = cudaSuccess;
+    void *p = nullptr;
+    if (need) e = cudaMalloc(&p, need);
+    if (e == cudaSuccess && need) {
+      blocks.push_back(p);
+      for (const Want &w : wanted) *w.out = static_cast<char *>(p) + w.off;
+      if (zero) e = cudaMemsetAsync(p, 0, need, st);
+    }
+    wanted.clear();
+    need = 0;
+    return e;
+  }
+  void free() {
+    for (void *p : blocks) cudaFree(p);
+    blocks.clear();
+  }
 };
 
 }  // namespace
@@ -141,6 +183,7 @@ struct mp_ctx {
   unsigned long long *h_kerr = nullptr;
   double *staging = nullptr;
   double *d_diag = nullptr;   // diagnostics scratch: per-plane partials, then the result
+  double *d_terms = nullptr;  // mp_objective's terms (kTerms doubles)
   double *h_diag = nullptr;   // pinned results (two doubles)
   size_t staging_n = 0;
   long long time = 0;
@@ -174,7 +217,9 @@ struct mp_ctx {
   // FP64 PLRC constants of the active poles: [D, dxi0, Crec][slot][re, im]
   double coef[3][3][2] = {{{0}}};
   double sumChi0 = 0, sumXi0 = 0;
-  std::vector<void *> allocs;
+  Arena mem;
+  void *pinned = nullptr;       // h_status, h_kerr, h_diag
+  std::vector<double> host_lines;  // the contents of `lines`
 };
 
 namespace {
@@ -199,15 +244,6 @@ int set_err(mp_ctx *c, int code, const char *fmt, ...) {
 int cuda_err(mp_ctx *c, cudaError_t e, const char *what) {
   return set_err(c, e == cudaErrorMemoryAllocation ? MP_ERR_NO_MEMORY : MP_ERR_CUDA, "%s: %s", what,
                  cudaGetErrorString(e));
-}
-
-cudaError_t dalloc(mp_ctx *c, void **p, size_t bytes) {
-  *p = nullptr;
-  if (bytes == 0) return cudaSuccess;
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) return e;
-  c->allocs.push_back(*p);
-  return cudaMemsetAsync(*p, 0, bytes, c->stream);
 }
 
 // Kappa lines exactly as CPMLBorder::initCoefficients (cpml_border.cpp:100-139)
@@ -514,9 +550,9 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
     if (e_ != cudaSuccess) return fail(cuda_err(c, e_, what)); \
   } while (0)
 
-  for (int f = 0; f < 6; ++f) MPB_TRY(dalloc(c, &c->F[f], c->fcount * c->esz), "field allocation");
+  for (int f = 0; f < 6; ++f) c->mem.want(&c->F[f], c->fcount * c->esz);
   if (g.plasma || g.plasma_current)
-    for (int q = 0; q < 4; ++q) MPB_TRY(dalloc(c, &c->plasma[q], c->fcount * c->esz), "plasma allocation");
+    for (int q = 0; q < 4; ++q) c->mem.want(&c->plasma[q], c->fcount * c->esz);
 
   const bool plrc = c->mode == MODE_PLRC_LIN || c->mode == MODE_PLRC_NONLIN;
   // PLRC: active poles (Delta eps != 0) and their accumulators over the medium
@@ -561,7 +597,7 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
     if (c->mz0 <= c->mz1) {
       c->psi_cells = size_t(c->mz1 - c->mz0 + 1) * size_t(c->plane);
       for (int s = 0; s < c->np; ++s)
-        for (int a = 0; a < 3; ++a) MPB_TRY(dalloc(c, &c->psi[s][a], 2 * c->psi_cells * c->esz), "psi allocation");
+        for (int a = 0; a < 3; ++a) c->mem.want(&c->psi[s][a], 2 * c->psi_cells * c->esz);
     }
   }
 
@@ -571,7 +607,7 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
   kappa_lines(g, kapE, kapH);
   const int n3[3] = {g.nx, g.ny, g.nz};
   const double d3[3] = {g.dx, g.dy, g.dz};
-  std::vector<double> host_lines;
+  std::vector<double> &host_lines = c->host_lines;
   std::vector<size_t> ikE_off(3), ikH_off(3);
   for (int a = 0; a < 3; ++a) {
     ikE_off[a] = host_lines.size();
@@ -636,8 +672,8 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
         L.n = size_t(L.ex) * L.ey * ez;
         if (L.n >= (size_t(1) << 31))
           return fail(set_err(c, MP_ERR_UNSUPPORTED, "CPML layer of %zu cells exceeds 2^31 (32-bit layer index)", L.n));
-        MPB_TRY(dalloc(c, &L.psi0, L.n * c->esz), "CPML allocation");
-        MPB_TRY(dalloc(c, &L.psi1, L.n * c->esz), "CPML allocation");
+        c->mem.want(&L.psi0, L.n * c->esz);
+        c->mem.want(&L.psi1, L.n * c->esz);
         L.b_off = host_lines.size();
         host_lines.insert(host_lines.end(), bl.begin(), bl.end());
         L.c_off = host_lines.size();
@@ -650,9 +686,7 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
   std::vector<double> wcoef(kFaddeevaTerms);
   double wL = 0;
   faddeeva_coefficients(wcoef.data(), &wL);
-  MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_wcoef), wcoef.size() * sizeof(double)), "source allocation");
-  MPB_TRY(cudaMemcpyAsync(c->d_wcoef, wcoef.data(), wcoef.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream),
-          "cudaMemcpy");
+  c->mem.want(&c->d_wcoef, wcoef.size() * sizeof(double));
   // All built injector kinds use the `down` face, and every injector on a face
   // shares the border-layer grids "IncidentEJx".. / "IncidentHJx".. of the first
   // one (Storage::addBorderLayer returns the grid already registered under the
@@ -718,7 +752,6 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
         p.sp_g = sp.g;
         p.tshift = q.t_shift;
         p.zshift = q.z_shift;
-        p.w_coef = c->d_wcoef;
         p.w_L = wL;
       }
     }
@@ -742,9 +775,9 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
     // plane pairs for up to 64 steps ahead, at most 256 MB
     const size_t per_step = 4 * size_t(c->plane) * c->esz;
     c->src_batch = int(std::max<size_t>(1, std::min<size_t>(64, (size_t(256) << 20) / per_step)));
-    MPB_TRY(dalloc(c, &c->src_buf, size_t(c->src_batch) * per_step), "source allocation");
+    c->mem.want(&c->src_buf, size_t(c->src_batch) * per_step);
     if (!c->gauss) {
-      MPB_TRY(dalloc(c, &c->src_buf2, size_t(c->src_batch) * per_step), "source allocation");
+      c->mem.want(&c->src_buf2, size_t(c->src_batch) * per_step);
       MPB_TRY(cudaStreamCreateWithFlags(&c->src_stream, cudaStreamNonBlocking), "cudaStreamCreate");
       for (int b = 0; b < 2; ++b) {
         MPB_TRY(cudaEventCreateWithFlags(&c->src_done[b], cudaEventDisableTiming), "cudaEventCreate");
@@ -752,9 +785,24 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
       }
     }
   }
+  c->mem.want(&c->lines, host_lines.size() * c->esz);
+  c->mem.want(&c->d_status, ST_COUNT * sizeof(int));
+  c->mem.want(&c->d_kerr, kKerrBytes);
+  c->mem.want(&c->d_diag, size_t(g.nz + 3) * sizeof(double));
+  c->mem.want(&c->d_terms, kTerms * sizeof(double));
+  const int *db = g.design_box;
+  c->design = db[0] <= db[1];
+  if (c->design) {
+    c->dcells = size_t(db[1] - db[0] + 1) * (db[3] - db[2] + 1) * (db[5] - db[4] + 1);
+    for (int a = 0; a < 3; ++a) c->mem.want(&c->d_design[a], c->dcells * sizeof(double));
+  }
+  MPB_TRY(c->mem.commit(c->stream, true), "device allocation");
 
+  for (int s = 0; s < c->nsrc; ++s)
+    for (int isH = 0; isH < 2; ++isH) c->sq[s][isH].w_coef = c->d_wcoef;
+  MPB_TRY(cudaMemcpyAsync(c->d_wcoef, wcoef.data(), wcoef.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream),
+          "cudaMemcpy");
   // upload the lines
-  MPB_TRY(dalloc(c, &c->lines, host_lines.size() * c->esz), "line allocation");
   if (c->fp32) {
     std::vector<float> hf(host_lines.begin(), host_lines.end());
     MPB_TRY(cudaMemcpyAsync(c->lines, hf.data(), hf.size() * 4, cudaMemcpyHostToDevice, c->stream), "cudaMemcpy");
@@ -764,29 +812,25 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
             "cudaMemcpy");
     MPB_TRY(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
   }
-  MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_status), ST_COUNT * sizeof(int)), "status allocation");
-  MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_status), ST_COUNT * sizeof(int)), "pinned allocation");
-  MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_kerr), kKerrBytes), "counter allocation");
-  MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_kerr), kKerrBytes), "pinned allocation");
-  MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_diag), size_t(g.nz + 3) * sizeof(double)), "diagnostics allocation");
-  MPB_TRY(cudaMallocHost(reinterpret_cast<void **>(&c->h_diag), 2 * sizeof(double)), "pinned allocation");
+  // the pinned results: the Kerr counters, two doubles, the status word
+  MPB_TRY(cudaMallocHost(&c->pinned, kKerrBytes + 2 * sizeof(double) + ST_COUNT * sizeof(int)), "pinned allocation");
+  c->h_kerr = static_cast<unsigned long long *>(c->pinned);
+  c->h_diag = reinterpret_cast<double *>(static_cast<char *>(c->pinned) + kKerrBytes);
+  c->h_status = reinterpret_cast<int *>(c->h_diag + 2);
 
   if (c->fp32) build_params<float>(c, c->epf, c->bpf, ikE_off, ikH_off, bzy_off, coef, numer, denom);
   else build_params<double>(c, c->epd, c->bpd, ikE_off, ikH_off, bzy_off, coef, numer, denom);
 
   // design region: FP64 maps with the defaults eps, 1, 1
-  if (g.design_box[0] <= g.design_box[1]) {
-    const int *db = g.design_box;
+  if (c->design) {
     DesignParams &d = c->dp;
     d.x0 = db[0] - 1; d.x1 = db[1] - 1;
     d.y0 = db[2] - 1; d.y1 = db[3] - 1;
     d.z0 = db[4]; d.z1 = db[5];
     d.bx = db[1] - db[0] + 1;
     d.by = db[3] - db[2] + 1;
-    c->dcells = size_t(d.bx) * d.by * (db[5] - db[4] + 1);
     const double init[3] = {g.eps, 1.0, 1.0};
     for (int a = 0; a < 3; ++a) {
-      MPB_TRY(dalloc(c, reinterpret_cast<void **>(&c->d_design[a]), c->dcells * sizeof(double)), "design allocation");
       std::vector<double> h(c->dcells, init[a]);
       MPB_TRY(cudaMemcpyAsync(c->d_design[a], h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream),
               "cudaMemcpy");
@@ -804,7 +848,6 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
     d.sumXi0 = c->sumXi0;
     d.chi = g.chi;
     d.lin = c->mode == MODE_PLRC_LIN;
-    c->design = true;
     if (c->fp32) c->epf.design = d;
     else c->epd.design = d;
   }
@@ -1244,15 +1287,13 @@ void mp_destroy(mp_ctx *c) {
     if (c->src_done[b]) cudaEventDestroy(c->src_done[b]);
     if (c->src_free[b]) cudaEventDestroy(c->src_free[b]);
   }
-  for (void *p : c->allocs) cudaFree(p);
+  c->mem.free();
   if (c->gauss) {
     gauss_destroy(*c->gauss);
     delete c->gauss;
   }
   if (c->staging) cudaFree(c->staging);
-  if (c->h_status) cudaFreeHost(c->h_status);
-  if (c->h_kerr) cudaFreeHost(c->h_kerr);
-  if (c->h_diag) cudaFreeHost(c->h_diag);
+  if (c->pinned) cudaFreeHost(c->pinned);
   free_host_ckpt(c);
   for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -1519,19 +1560,11 @@ namespace {
 // Device buffers of one call, freed (after the stream drains) when it returns.
 struct DevBufs {
   cudaStream_t st;
-  std::vector<void *> p;
+  Arena mem;
   explicit DevBufs(cudaStream_t s) : st(s) {}
   ~DevBufs() {
     cudaStreamSynchronize(st);
-    for (void *q : p) cudaFree(q);
-  }
-  cudaError_t alloc(void **out, size_t bytes) {
-    *out = nullptr;
-    if (!bytes) return cudaSuccess;
-    cudaError_t e = cudaMalloc(out, bytes);
-    if (e != cudaSuccess) return e;
-    p.push_back(*out);
-    return cudaMemsetAsync(*out, 0, bytes, st);
+    mem.free();
   }
 };
 
@@ -1554,9 +1587,12 @@ std::vector<std::pair<void *, size_t>> state_regions(const mp_ctx *c) {
 
 // The adjoint face entry per axis of the E (isH false) or H CPML currents: the
 // low and the high face of the axis together (their layers must not overlap,
-// so that a cell is in at most one face per axis).
+// so that a cell is in at most one face per axis).  Its arrays are noted in buf;
+// coefficient lines of two faces are appended to `lines`, and where each belongs
+// to `merged`.
 template <typename T>
-int adj_faces(mp_ctx *c, DevBufs &buf, bool isH, const CpmlFace<T> *fw, AdjFace<T> out[3]) {
+int adj_faces(mp_ctx *c, DevBufs &buf, bool isH, const CpmlFace<T> *fw, AdjFace<T> out[3], std::vector<T> &lines,
+              std::vector<std::pair<const T **, size_t>> &merged) {
   const mp_config &g = c->cfg;
   const int n3[3] = {g.nx, g.ny, g.nz};
   for (int dim = 0; dim < 3; ++dim) {
@@ -1591,12 +1627,8 @@ int adj_faces(mp_ctx *c, DevBufs &buf, bool isH, const CpmlFace<T> *fw, AdjFace<
     const size_t cells = dim == 2 ? size_t(ntot) * size_t(c->plane) : zdepth * size_t(F.ex) * size_t(F.ey);
     if (cells >= (size_t(1) << 31))  // the adjoint kernels index face arrays in 32 bits
       return set_err(c, MP_ERR_UNSUPPORTED, "mp_adjoint: CPML face array of %zu cells exceeds 2^31", cells);
-    void *a0, *a1;
-    cudaError_t e;
-    if ((e = buf.alloc(&a0, cells * sizeof(T))) != cudaSuccess || (e = buf.alloc(&a1, cells * sizeof(T))) != cudaSuccess)
-      return cuda_err(c, e, "adjoint allocation");
-    F.a0 = static_cast<T *>(a0);
-    F.a1 = static_cast<T *>(a1);
+    buf.mem.want(&F.a0, cells * sizeof(T));
+    buf.mem.want(&F.a1, cells * sizeof(T));
     F.n = (long long)cells;
     if (!B) {
       F.b = fw[fa].b;
@@ -1604,25 +1636,12 @@ int adj_faces(mp_ctx *c, DevBufs &buf, bool isH, const CpmlFace<T> *fw, AdjFace<
       continue;
     }
     // the two faces' b and c lines are zero outside their layers: add them
+    // (the low face's in A, the high one's in B)
     const size_t len = size_t(n3[dim]) + 2;
-    std::vector<T> hb(len), hc(len), tb(len), tc(len);
-    if ((e = cudaMemcpy(hb.data(), fw[fa].b, len * sizeof(T), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-        (e = cudaMemcpy(hc.data(), fw[fa].c, len * sizeof(T), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-        (e = cudaMemcpy(tb.data(), fw[fb].b, len * sizeof(T), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-        (e = cudaMemcpy(tc.data(), fw[fb].c, len * sizeof(T), cudaMemcpyDeviceToHost)) != cudaSuccess)
-      return cuda_err(c, e, "line read");
-    for (size_t q = 0; q < len; ++q) {
-      hb[q] += tb[q];
-      hc[q] += tc[q];
-    }
-    void *lb, *lc;
-    if ((e = buf.alloc(&lb, len * sizeof(T))) != cudaSuccess || (e = buf.alloc(&lc, len * sizeof(T))) != cudaSuccess ||
-        (e = cudaMemcpyAsync(lb, hb.data(), len * sizeof(T), cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(lc, hc.data(), len * sizeof(T), cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
-      return cuda_err(c, e, "line upload");
-    F.b = static_cast<const T *>(lb);
-    F.c = static_cast<const T *>(lc);
+    merged.push_back({&F.b, lines.size()});
+    for (size_t q = 0; q < len; ++q) lines.push_back(T(c->host_lines[A->b_off + q]) + T(c->host_lines[B->b_off + q]));
+    merged.push_back({&F.c, lines.size()});
+    for (size_t q = 0; q < len; ++q) lines.push_back(T(c->host_lines[A->c_off + q]) + T(c->host_lines[B->c_off + q]));
   }
   return MP_OK;
 }
@@ -1688,8 +1707,13 @@ template <typename T>
 int objective_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_config *a, double *J) {
   DevBufs buf(c->stream);
   double *terms;
-  cudaError_t e = buf.alloc(reinterpret_cast<void **>(&terms), (size_t(a->steps) * objective_parts(a) + 1) * sizeof(double));
+  // the context's buffer where the terms fit in it (an allocation and its release
+  // cost 0.65 ms a call)
+  const size_t n = size_t(a->steps) * objective_parts(a) + 1;
+  if (n > kTerms) buf.mem.want(&terms, n * sizeof(double));
+  cudaError_t e = buf.mem.commit(c->stream, false);
   if (e != cudaSuccess) return cuda_err(c, e, "objective allocation");
+  if (n <= kTerms) terms = c->d_terms;
   StepHooks h;
   h.after = [&](long long n) { return objective_term<T>(c, a, terms, n); };
   int rc = step_impl<T>(c, ep, bp, a->steps, nullptr, nullptr, &h);
@@ -1957,13 +1981,17 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
     hist[1] = rec->hist[1];
     terms = rec->terms;
   } else {
-    if ((e = sbuf.alloc(reinterpret_cast<void **>(&ckpt), size_t(slots + 1) * S)) != cudaSuccess ||
-        (e = sbuf.alloc(reinterpret_cast<void **>(&hist[0]), size_t(K + 1) * H)) != cudaSuccess ||
-        (e = sbuf.alloc(reinterpret_cast<void **>(&terms), (size_t(Tn) * objective_parts(a) + 1) * sizeof(double))) != cudaSuccess)
-      return cuda_err(c, e, "checkpoint allocation");
-    if (nbuf == 2 && sbuf.alloc(reinterpret_cast<void **>(&hist[1]), size_t(K + 1) * H) != cudaSuccess) {
-      cudaGetLastError();  // no room for the second buffer: chunks run forward and back in turn
-      nbuf = 1;
+    // written before they are read: not zeroed
+    sbuf.mem.want(&ckpt, size_t(slots + 1) * S);
+    sbuf.mem.want(&hist[0], size_t(K + 1) * H);
+    sbuf.mem.want(&terms, (size_t(Tn) * objective_parts(a) + 1) * sizeof(double));
+    if ((e = sbuf.mem.commit(c->stream, false)) != cudaSuccess) return cuda_err(c, e, "checkpoint allocation");
+    if (nbuf == 2) {
+      sbuf.mem.want(&hist[1], size_t(K + 1) * H);
+      if (sbuf.mem.commit(c->stream, false) != cudaSuccess) {
+        cudaGetLastError();  // no room for the second buffer: chunks run forward and back in turn
+        nbuf = 1;
+      }
     }
   }
   // The reverse pass runs on a second stream: the adjoint kernels of one chunk
@@ -1992,33 +2020,31 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
       return cuda_err(c, e, "cudaEventCreate");
   int cur = 0;  // history buffer of the chunk being run forward
   AdjParams<T> p = AdjParams<T>();
-  for (int q = 0; q < 3 && phase != kAdjRecord; ++q) {
-    void *eb, *bb, *gg;
-    double *gr;
-    if ((e = buf.alloc(&eb, fbytes)) != cudaSuccess || (e = buf.alloc(&bb, fbytes)) != cudaSuccess ||
-        (e = buf.alloc(&gg, fbytes)) != cudaSuccess ||
-        (e = buf.alloc(reinterpret_cast<void **>(&gr), c->dcells * sizeof(double))) != cudaSuccess)
-      return cuda_err(c, e, "adjoint allocation");
-    p.Eb[q] = static_cast<T *>(eb);
-    p.Bb[q] = static_cast<T *>(bb);
-    p.G[q] = static_cast<T *>(gg);
-    p.grad[q] = gr;
-  }
-  for (int s = 0; s < c->np && phase != kAdjRecord; ++s)
-    for (int q = 0; q < 3; ++q) {
-      void *ps;
-      if ((e = buf.alloc(&ps, 2 * c->psi_cells * sizeof(T))) != cudaSuccess) return cuda_err(c, e, "adjoint allocation");
-      p.psib[s][q] = static_cast<T *>(ps);
-    }
   if (phase != kAdjRecord) {
-    void *dp = nullptr;
-    if (c->np > 0 && (e = buf.alloc(&dp, c->dcells * c->np * 6 * sizeof(T))) != cudaSuccess)
-      return cuda_err(c, e, "adjoint allocation");
-    p.dpsi = static_cast<T *>(dp);
-  }
-  for (int isH = 0; isH < 2 && phase != kAdjRecord; ++isH) {
-    const int rc = adj_faces<T>(c, buf, isH != 0, isH ? bp.cpml : ep.cpml, isH ? p.fh : p.fe);
-    if (rc != MP_OK) return rc;
+    for (int q = 0; q < 3; ++q) {
+      buf.mem.want(&p.Eb[q], fbytes);
+      buf.mem.want(&p.Bb[q], fbytes);
+      buf.mem.want(&p.G[q], fbytes);
+      buf.mem.want(&p.grad[q], c->dcells * sizeof(double));
+    }
+    for (int s = 0; s < c->np; ++s)
+      for (int q = 0; q < 3; ++q) buf.mem.want(&p.psib[s][q], 2 * c->psi_cells * sizeof(T));
+    buf.mem.want(&p.dpsi, c->dcells * c->np * 6 * sizeof(T));
+    std::vector<T> lines;  // coefficient lines of the axes with two faces
+    std::vector<std::pair<const T **, size_t>> merged;
+    for (int isH = 0; isH < 2; ++isH) {
+      const int rc = adj_faces<T>(c, buf, isH != 0, isH ? bp.cpml : ep.cpml, isH ? p.fh : p.fe, lines, merged);
+      if (rc != MP_OK) return rc;
+    }
+    T *dlines;
+    buf.mem.want(&dlines, lines.size() * sizeof(T));
+    if ((e = buf.mem.commit(c->stream, true)) != cudaSuccess) return cuda_err(c, e, "adjoint allocation");
+    if (!lines.empty() &&
+        ((e = cudaMemcpyAsync(dlines, lines.data(), lines.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream)) !=
+             cudaSuccess ||
+         (e = cudaStreamSynchronize(c->stream)) != cudaSuccess))
+      return cuda_err(c, e, "line upload");
+    for (const auto &m : merged) *m.first = dlines + m.second;
   }
   p.nx = g.nx; p.ny = g.ny; p.nz = g.nz;
   p.status = c->d_status;
@@ -2086,9 +2112,16 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
   p.chi_nl_t = T(p.nonlin ? p.chi : 0.0);
   p.obj_f_t = T(p.obj_f);
 
+  // the state's arrays that lie one after the other in memory, copied together
+  std::vector<std::pair<void *, size_t>> runs;
+  for (const auto &r : regions)
+    if (!runs.empty() && static_cast<char *>(runs.back().first) + runs.back().second == r.first)
+      runs.back().second += r.second;
+    else
+      runs.push_back(r);
   auto copy_state = [&](long long slot, bool save) -> cudaError_t {
     size_t off = 0;
-    for (const auto &r : regions) {
+    for (const auto &r : runs) {
       char *ck = ckpt + size_t(slot) * S + off;
       cudaError_t err = save ? cudaMemcpyAsync(ck, r.first, r.second, cudaMemcpyDeviceToDevice, c->stream)
                              : cudaMemcpyAsync(r.first, ck, r.second, cudaMemcpyDeviceToDevice, c->stream);
@@ -2270,7 +2303,7 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
     // the live state to / from the host copy of segment k, on the stream
     auto host_copy = [&](long long k, bool save) -> cudaError_t {
       size_t off = 0;
-      for (const auto &r : regions) {
+      for (const auto &r : runs) {
         char *hc = static_cast<char *>(c->host_ckpt[size_t(k)]) + off;
         cudaError_t err = save ? cudaMemcpyAsync(hc, r.first, r.second, cudaMemcpyDeviceToHost, c->stream)
                                : cudaMemcpyAsync(r.first, hc, r.second, cudaMemcpyHostToDevice, c->stream);
