@@ -32,103 +32,54 @@
 // warp do not cover the latency of HBM: the next plane's lines are prefetched
 // into L2 while this plane is computed, which needs no registers.
 // Measured per half step, before -> after (B200, us):
-//   256 x 256 x 512 PLRC + Kerr FP32   E 758 -> 681   B 276 -> 258
-//   192 x 192 x 384 PLRC + Kerr FP64   E 659 -> 551   B 225 -> 198
-//   150 x 131 x 210 fdtd-plain FP32    E  37 ->  30   B  48 ->  31
-//   101 x 75 x 163 fdtd-nl FP64        E  49 ->  26   B  40 ->  17
-//   128 x 128 x 192 + plasma FP32      E 135 -> 109   B  56 ->  43
+//   256 x 256 x 512 PLRC + Kerr FP32   E 758 -> 666   B 276 -> 250
+//   192 x 192 x 384 PLRC + Kerr FP64   E 659 -> 547   B 225 -> 199
+//   150 x 131 x 210 fdtd-plain FP32    E  37 ->  28   B  48 ->  29
+//   101 x 75 x 163 fdtd-nl FP64        E  49 ->  24   B  40 ->  16
+//   128 x 128 x 192 + plasma FP32      E 135 -> 106   B  56 ->  37
 #include "mp_cell.cuh"
 #include "mp_pdl.cuh"
+#include "mp_row.cuh"
 
 #include <algorithm>
 
-// Resident threads per SM asked of the register allocator.  E half: FP32 with
-// one cell per thread 1024 (64 registers; 768 lets the compiler take 75 with the
-// plasma plug-ins: 114 instead of 109 us on 128 x 128 x 192), with two cells 768
-// (80 registers); FP64 640 (96 registers; 768 spill: 96 instead of 87 us with a
-// design region, 120 x 104 x 136).  B half: FP32 1280 (48 registers; 1024: 264
-// instead of 257 us on 256 x 256 x 512), FP64 768 (640: 205, 1024: 206, 768:
-// 198 us on 192 x 192 x 384).
-#ifndef MPB_E_THREADS_F
-#define MPB_E_THREADS_F 1024
-#endif
-#ifndef MPB_E_THREADS_F2
-#define MPB_E_THREADS_F2 768
-#endif
-#ifndef MPB_E_THREADS_D
-#define MPB_E_THREADS_D 640
-#endif
-#ifndef MPB_B_THREADS_F
-#define MPB_B_THREADS_F 1280
-#endif
-#ifndef MPB_B_THREADS_D
-#define MPB_B_THREADS_D 768
-#endif
-
 namespace mpb {
 
-// Rows (warps) per block: with one row the y neighbours come from other blocks
-// through L2 and the 256 x 256 x 512 E half takes 824 instead of 737 us; 2 and 8
-// rows 1% and 7% slower than 4.
-constexpr int kRowTile = 4;
-constexpr int kRowThreads = 32 * kRowTile;
+// Resident threads per SM asked of the register allocator.  E half: FP32 with
+// one cell per thread 1024 (64 registers; 896: 687 instead of 666 us on 256 x 256 x
+// 512), with the plasma plug-ins 896 (106 instead of 114 us on 128 x 128 x 192),
+// with two cells 768 (80 registers); FP64 640 (96 registers; 768 spill: 96
+// instead of 87 us with a design region, 120 x 104 x 136).  B half: FP32 1280 (48
+// registers; 1024: 264 instead of 257 us on 256 x 256 x 512), with the faces
+// loaded early 768 (80 registers; 1024: 263 instead of 250), FP64 768 (640: 205,
+// 1024: 206, 768: 198 us on 192 x 192 x 384).
+template <typename T>
+__host__ __device__ constexpr int e_threads(int V, bool plasma) {
+  return sizeof(T) == 8 ? 640 : V == 2 ? 768 : plasma ? 896 : 1024;
+}
+template <typename T>
+__host__ __device__ constexpr int b_threads(bool early) {
+  return sizeof(T) == 8 ? 768 : early ? 768 : 1280;
+}
 
 __device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
-// V consecutive elements of a row.
-template <typename T, int V>
-struct alignas(sizeof(T) * V <= 16 ? sizeof(T) * V : 16) RowV {
-  T v[V];
-};
-
-// The accesses at column c of the plane at element `base` of an array of n
-// elements (aligned to a row of V), checked like ld_c / st_c.  Plain loads, not
-// the read-only path: a kernel launched early must not have them moved ahead
-// of its wait.
-template <typename T, int V>
-__device__ __forceinline__ bool row_in(long long i, long long n, int *st) {
-  return in_bounds(i, n, st) && (V == 1 || in_bounds(i + V - 1, n, st));
-}
-template <int V, typename T>
-__device__ __forceinline__ RowV<T, V> ldp(const T *a, long long base, unsigned c, long long n, int *st) {
-  RowV<T, V> r = {};
-  if (row_in<T, V>(base + c, n, st)) r = *reinterpret_cast<const RowV<T, V> *>(a + base + c);
-  return r;
-}
-template <int V, typename T>
-__device__ __forceinline__ void stp(T *a, long long base, unsigned c, long long n, int *st, const RowV<T, V> &r) {
-  if (row_in<T, V>(base + c, n, st)) *reinterpret_cast<RowV<T, V> *>(a + base + c) = r;
-}
-
-// The columns of a thread, row j, columns i0 .. i0 + V - 1 of the plane: rows
-// are taken in groups of kRowTile, warp w of a block holds row w of a group, and
-// its 32 lanes run along the row and on into the same row of the next group, so
-// that a block covers kRowTile neighbouring rows (their y neighbours meet in
-// L1) and no lane is idle on narrow or odd rows.
-struct RowGrid {
-  unsigned nrow, nvec;  // threads per row (nx / V), and per warp over all groups
-  unsigned mul, shift;  // t / nrow = (t * mul) >> (32 + shift) for t < 2^31
+// What a half step's grid needs beside the row mapping.
+struct HalfGrid : RowMap {
   int kchunk;           // planes per block
   int ahead;            // prefetch the next plane into L2
   // the CPML layers: cells with MPulse index <= lo[a] or >= hi[a] along axis a
   // lie in a layer
   int lo[3], hi[3];
   int src;              // the injection plane (-1: none)
+  // there are x / y layers, and no thread's cells reach into both layers of an axis
+  bool apart;
 };
-
-template <int V>
-__device__ __forceinline__ bool row_cells(const RowGrid &g, int ny, int &i0, int &j) {
-  const unsigned t = blockIdx.x * 32 + (threadIdx.x & 31);
-  const unsigned grp = __umulhi(t, g.mul) >> g.shift;
-  i0 = int(t - grp * g.nrow) * V;
-  j = int(grp * kRowTile + (threadIdx.x >> 5));
-  return t < g.nvec && j < ny;
-}
 
 // Bits of the x faces (slots 2 high, 3 low) at the V cells of a thread, bits 2c
 // and 2c + 1, and of the y faces (slots 0 high, 1 low), bits 2V and 2V + 1.
 template <int V>
-__device__ __forceinline__ unsigned row_face_mask(const RowGrid &g, int i0, int j) {
+__device__ __forceinline__ unsigned row_face_mask(const HalfGrid &g, int i0, int j) {
   unsigned m = (j + 1 >= g.hi[1] ? 1u << (2 * V) : 0u) | (j + 1 <= g.lo[1] ? 2u << (2 * V) : 0u);
 #pragma unroll
   for (int c = 0; c < V; ++c)
@@ -194,6 +145,110 @@ __device__ __forceinline__ void face_currents(const CpmlFace<T> (&cpml)[6], int 
   if (zlow) face_row<T, V, 5>(cpml[5], nx, ny, i0, j, k, 0, dz0, dz1, cur, st);
 }
 
+// The same for grids whose layers lie apart (HalfGrid::apart: a thread's cells
+// are in at most one face per axis), in two parts: load_faces asks for the psi
+// and coefficients of all faces of the plane beside the plane's other loads, so
+// that a face costs no memory latency of its own; add_faces then does the rest,
+// in the same order.  face_currents waits once per face, and a warp with x-face
+// cells does so on every plane.  B half with CPML on all faces (FP32, us): 96^3
+// 18.8 -> 14.1, 128 x 128 x 192 44 -> 37, 128 x 128 x 256 54 -> 45, 256 x 256 x 512
+// 260 -> 250; E half 128 x 128 x 256 Kerr 107 -> 102, 256 x 256 x 512 676 -> 666,
+// 101 x 131 x 120 with two poles 49 -> 43, FP64 120 x 104 x 136 87 -> 82.  Grids
+// without x / y layers keep face_currents, which needs fewer registers (160 x 144
+// x 250 with z layers, B half 44 us; with the early loads 50), and so do grids
+// whose layers meet.
+template <typename T, int V>
+struct FaceRows {
+  RowV<T, V> y0, y1, z0, z1;
+  T x0[V], x1[V];
+  T by, cy, bz, cz, bx[V], cx[V];
+  unsigned ly, lz;
+  int lx;
+};
+
+template <typename T, int V>
+__device__ __forceinline__ void load_faces(const CpmlFace<T> (&cpml)[6], int nx, int ny, unsigned mask, bool zlow,
+                                           bool zhigh, int i0, int j, int k, FaceRows<T, V> &f, int *st) {
+  constexpr unsigned kX = (1u << (2 * V)) - 1u;
+  if (mask) {
+    if (mask & ~kX) {
+      const CpmlFace<T> &L = cpml[(mask >> (2 * V)) & 1u ? 0 : 1];
+      f.ly = unsigned(((k - L.zlo) * L.ey + (j + 1 - L.lo)) * nx + i0);
+      f.by = ld(L.b + j + 1);
+      f.cy = ld(L.c + j + 1);
+      f.y0 = ldp<V>(L.psi0, 0, f.ly, L.n, st);
+      f.y1 = ldp<V>(L.psi1, 0, f.ly, L.n, st);
+    }
+    if (mask & kX) {
+      const CpmlFace<T> &L = cpml[mask & (0x55555555u & kX) ? 2 : 3];
+      f.lx = ((k - L.zlo) * ny + j) * L.ex + (i0 + 1 - L.lo);
+#pragma unroll
+      for (int c = 0; c < V; ++c)
+        if (mask & (3u << (2 * c))) {
+          f.bx[c] = ld(L.b + i0 + c + 1);
+          f.cx[c] = ld(L.c + i0 + c + 1);
+          f.x0[c] = ld_c(L.psi0, f.lx + c, L.n, st);
+          f.x1[c] = ld_c(L.psi1, f.lx + c, L.n, st);
+        }
+    }
+  }
+  if (zlow || zhigh) {
+    const CpmlFace<T> &L = cpml[zhigh ? 4 : 5];
+    f.lz = unsigned(((k - L.lo) * ny + j) * nx + i0);
+    f.bz = ld(L.b + k);
+    f.cz = ld(L.c + k);
+    f.z0 = ldp<V>(L.psi0, 0, f.lz, L.n, st);
+    f.z1 = ldp<V>(L.psi1, 0, f.lz, L.n, st);
+  }
+}
+
+template <typename T, int V>
+__device__ __forceinline__ void add_faces(const CpmlFace<T> (&cpml)[6], unsigned mask, bool zlow, bool zhigh,
+                                          FaceRows<T, V> &f, const T (&dy0)[V], const T (&dy1)[V], const T (&dx0)[V],
+                                          const T (&dx1)[V], const T (&dz0)[V], const T (&dz1)[V], T (&cur)[V][3],
+                                          int *st) {
+  constexpr unsigned kX = (1u << (2 * V)) - 1u;
+  if (mask) {
+    if (mask & ~kX) {
+      const CpmlFace<T> &L = cpml[(mask >> (2 * V)) & 1u ? 0 : 1];
+#pragma unroll
+      for (int c = 0; c < V; ++c) {
+        f.y0.v[c] = fma_pp(f.by, f.y0.v[c], f.cy, dy0[c]);
+        f.y1.v[c] = fma_pp(f.by, f.y1.v[c], f.cy, dy1[c]);
+        cur[c][2] += f.y0.v[c];
+        cur[c][0] += f.y1.v[c];
+      }
+      stp<V>(L.psi0, 0, f.ly, L.n, st, f.y0);
+      stp<V>(L.psi1, 0, f.ly, L.n, st, f.y1);
+    }
+    if (mask & kX) {
+      const CpmlFace<T> &L = cpml[mask & (0x55555555u & kX) ? 2 : 3];
+#pragma unroll
+      for (int c = 0; c < V; ++c)
+        if (mask & (3u << (2 * c))) {
+          const T p0 = fma_pp(f.bx[c], f.x0[c], f.cx[c], dx0[c]);
+          const T p1 = fma_pp(f.bx[c], f.x1[c], f.cx[c], dx1[c]);
+          st_c(L.psi0, f.lx + c, L.n, st, p0);
+          st_c(L.psi1, f.lx + c, L.n, st, p1);
+          cur[c][1] += p0;
+          cur[c][2] += p1;
+        }
+    }
+  }
+  if (zlow || zhigh) {
+    const CpmlFace<T> &L = cpml[zhigh ? 4 : 5];
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      f.z0.v[c] = fma_pp(f.bz, f.z0.v[c], f.cz, dz0[c]);
+      f.z1.v[c] = fma_pp(f.bz, f.z1.v[c], f.cz, dz1[c]);
+      cur[c][0] += f.z0.v[c];
+      cur[c][1] += f.z1.v[c];
+    }
+    stp<V>(L.psi0, 0, f.lz, L.n, st, f.z0);
+    stp<V>(L.psi1, 0, f.lz, L.n, st, f.z1);
+  }
+}
+
 // The injection plane's currents of the V cells.
 template <typename T, int V, typename P>
 __device__ __forceinline__ void source_currents(const P &p, unsigned col, T (&cur)[V][3]) {
@@ -219,15 +274,15 @@ __device__ __forceinline__ bool hist_cell(const EParams<T> &p, int i, int j, int
   return false;
 }
 
-template <typename T, int V, int MODE, int NP, bool DESIGN, bool PLASMA>
-__global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 8 ? MPB_E_THREADS_D : V == 1 ? MPB_E_THREADS_F : MPB_E_THREADS_F2) / kRowThreads)
-    e_half_kernel(const EParams<T> p, const RowGrid g) {
+template <typename T, int V, int MODE, int NP, bool DESIGN, bool PLASMA, bool EARLY>
+__global__ void __launch_bounds__(kRowThreads, e_threads<T>(V, PLASMA) / kRowThreads)
+    e_half_kernel(const EParams<T> p, const HalfGrid g) {
   typedef typename Vec2<T>::type T2;
   constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
   pdl_launch_dependents();
   const int nx = p.nx, ny = p.ny;
   int i0, j;  // 0-based: MPulse i + 1, j + 1
-  if (!row_cells<V>(g, ny, i0, j)) return;
+  if (!row_cells<V>(g, blockIdx.x, ny, i0, j)) return;
   const int k0 = p.k_first + blockIdx.y * g.kchunk;
   const int k1 = min(k0 + g.kchunk - 1, p.k_last);
   const long long plane = p.plane;
@@ -278,6 +333,9 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 8 ? MPB_E_THREADS_D
       }
     }
     const T ikz = ld(p.ik[2] + k);
+    const bool zlow = PLRC && k <= g.lo[2], zhigh = PLRC && k >= g.hi[2];
+    FaceRows<T, V> fr;
+    if (PLRC && EARLY) load_faces<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, fr, st);
     if (g.ahead && k < k1) {
       const long long ba = base + plane;
       prefetch_l2(Bx + ba + col);
@@ -310,7 +368,6 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 8 ? MPB_E_THREADS_D
 #pragma unroll
     for (int c = 0; c < V; ++c) cur[c][0] = cur[c][1] = cur[c][2] = T(0);
     if (PLRC) {
-      const bool zlow = k <= g.lo[2], zhigh = k >= g.hi[2];
       if (fmask || zlow || zhigh) {
         T nxy[V], nzx[V], nyz[V];
 #pragma unroll
@@ -319,7 +376,10 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 8 ? MPB_E_THREADS_D
           nzx[c] = -dzx[c];
           nyz[c] = -dyz[c];
         }
-        face_currents<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, nxy, dzy, nzx, dyx, nyz, dxz, cur, st);
+        if (EARLY)
+          add_faces<T, V>(p.cpml, fmask, zlow, zhigh, fr, nxy, dzy, nzx, dyx, nyz, dxz, cur, st);
+        else
+          face_currents<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, nxy, dzy, nzx, dyx, nyz, dxz, cur, st);
       }
       if (k == g.src) source_currents<T, V>(p, col, cur);
     }
@@ -392,16 +452,16 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 8 ? MPB_E_THREADS_D
   flush_kerr_count<MODE>(p.kerr_count, kc);
 }
 
-template <typename T, int V>
-__global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F : MPB_B_THREADS_D) / kRowThreads)
-    b_half_kernel(const BParams<T> p, const RowGrid g) {
+template <typename T, int V, bool EARLY>
+__global__ void __launch_bounds__(kRowThreads, b_threads<T>(EARLY) / kRowThreads)
+    b_half_kernel(const BParams<T> p, const HalfGrid g) {
   // the chunks from the top down: the E half wrote the top planes last, and
   // what of them is still in L2 is read from there (2-6% of both halves on grids
   // of up to twice the L2)
   pdl_launch_dependents();
   const int nx = p.nx, ny = p.ny;
   int i0, j;
-  if (!row_cells<V>(g, ny, i0, j)) return;
+  if (!row_cells<V>(g, blockIdx.x, ny, i0, j)) return;
   const int k0 = p.k_first + (gridDim.y - 1 - blockIdx.y) * g.kchunk;
   const int k1 = min(k0 + g.kchunk - 1, p.k_last);
   const long long plane = p.plane;
@@ -433,6 +493,9 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F
     const RowV<T, V> ez_yp = ldp<V>(Ez, base, colyp, nf, st), ex_yp = ldp<V>(Ex, base, colyp, nf, st);
     const RowV<T, 1> ez_xl = ldp<1>(Ez, base, colxp, nf, st), ey_xl = ldp<1>(Ey, base, colxp, nf, st);
     const T ikz = ld(p.ik[2] + k);
+    const bool zlow = k <= g.lo[2], zhigh = k >= g.hi[2];
+    FaceRows<T, V> fr;
+    if (EARLY) load_faces<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, fr, st);
     if (g.ahead && k < k1) {
       const long long ba = base + plane;
       prefetch_l2(Bx + ba + col);
@@ -457,7 +520,6 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F
     T cur[V][3];
 #pragma unroll
     for (int c = 0; c < V; ++c) cur[c][0] = cur[c][1] = cur[c][2] = T(0);
-    const bool zlow = k <= g.lo[2], zhigh = k >= g.hi[2];
     if (fmask || zlow || zhigh) {
       T nzy[V], nyx[V], nxz[V];
 #pragma unroll
@@ -466,7 +528,10 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F
         nyx[c] = -dyx[c];
         nxz[c] = -dxz[c];
       }
-      face_currents<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, dxy, nzy, dzx, nyx, dyz, nxz, cur, st);
+      if (EARLY)
+        add_faces<T, V>(p.cpml, fmask, zlow, zhigh, fr, dxy, nzy, dzx, nyx, dyz, nxz, cur, st);
+      else
+        face_currents<T, V>(p.cpml, nx, ny, fmask, zlow, zhigh, i0, j, k, dxy, nzy, dzx, nyx, dyz, nxz, cur, st);
     }
     if (k == g.src) source_currents<T, V>(p, col, cur);
 
@@ -489,6 +554,11 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F
 // ---------------------------------------------------------------------------
 // Launchers (called from mp_api.cu)
 
+template <typename P>
+static bool xy_faces(const P &p) {
+  return p.cpml[0].active || p.cpml[1].active || p.cpml[2].active || p.cpml[3].active;
+}
+
 // The grid of a half step: V cells per thread, z-chunks of the planes.
 // Planes per block: one where two would leave SMs without four blocks (32^3
 // FP64: E 9.1 instead of 10.2 us); else at least two, and more while 50 blocks
@@ -499,22 +569,16 @@ __global__ void __launch_bounds__(kRowThreads, (sizeof(T) == 4 ? MPB_B_THREADS_F
 // states that do not stay in L2 (126 MB): 256 x 256 x 512 E half 748 -> 677 us,
 // 120 x 104 x 136 FP64 93 -> 89; on a 99 MB state 29.8 -> 31.5.
 template <typename P>
-static RowGrid row_grid(const P &p, int V, int max_planes, dim3 *d) {
-  RowGrid r;
-  r.nrow = unsigned(p.nx / V);
-  r.nvec = r.nrow * unsigned((p.ny + kRowTile - 1) / kRowTile);
-  // nrow >= 2; exact for every t < 2^31 with shift = ceil(log2(nrow)) - 1 and
-  // mul = ceil(2^(32 + shift) / nrow) (Granlund and Montgomery, PLDI 1994)
-  int l = 0;
-  while ((1ULL << l) < r.nrow) ++l;
-  r.shift = unsigned(l - 1);
-  r.mul = unsigned(((1ULL << (32 + r.shift)) + r.nrow - 1) / r.nrow);
+static HalfGrid row_grid(const P &p, int V, int max_planes, dim3 *d) {
+  HalfGrid r;
+  static_cast<RowMap &>(r) = row_map(p.nx, p.ny, V);
   const int axis_high[3] = {2, 0, 4};  // the slot of the high face; the low one follows
   for (int a = 0; a < 3; ++a) {
     const auto &H = p.cpml[axis_high[a]], &L = p.cpml[axis_high[a] + 1];
     r.hi[a] = H.active ? H.lo : 1 << 30;
     r.lo[a] = L.active ? L.hi : -1;
   }
+  r.apart = xy_faces(p) && r.hi[0] - r.lo[0] > V && r.hi[1] > r.lo[1] && r.hi[2] > r.lo[2];
   r.src = p.n_src > 0 ? p.src[0].plane : -1;
   const int nk = p.k_last - p.k_first + 1;
   const long long bxy = (r.nvec + 31) / 32, all = bxy * nk;
@@ -532,29 +596,39 @@ constexpr int max_planes() {
   return sizeof(T) == 4 ? 8 : 4;
 }
 
+template <typename T, int V, int MODE, bool DESIGN, bool PLASMA, bool EARLY>
+static cudaError_t launch_e_np(const EParams<T> &p, int np, const HalfGrid &g, dim3 d, cudaStream_t st) {
+  constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
+  const dim3 b(kRowThreads, 1, 1);
+  switch (PLRC ? np : 0) {
+    case 0: return launch_pdl(e_half_kernel<T, V, MODE, 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+    case 1: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 1 : 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+    case 2: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 2 : 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+    default: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 3 : 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+  }
+}
+
 template <typename T, int V, int MODE, bool DESIGN, bool PLASMA>
 static cudaError_t launch_e_v(const EParams<T> &p, int np, cudaStream_t st) {
   constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
   dim3 d;
-  const RowGrid g = row_grid(p, V, max_planes<T>(), &d);
-  switch (PLRC ? np : 0) {
-    case 0: return launch_pdl(e_half_kernel<T, V, MODE, 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
-    case 1: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 1 : 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
-    case 2: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 2 : 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
-    default: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 3 : 0, DESIGN, PLASMA>, d, dim3(kRowThreads, 1, 1), st, p, g);
-  }
+  const HalfGrid g = row_grid(p, V, max_planes<T>(), &d);
+  return PLRC && g.apart ? launch_e_np<T, V, MODE, DESIGN, PLASMA, PLRC>(p, np, g, d, st)
+                         : launch_e_np<T, V, MODE, DESIGN, PLASMA, false>(p, np, g, d, st);
 }
 
 // Two cells per thread in FP32 where the update is short (150 x 131 x 210
 // fdtd-plain 30 instead of 38 us, 160 x 144 x 250 PLRC with one pole 79 instead
-// of 81, 128^3 with two poles 46 instead of 49); one with Kerr or the plasma
+// of 81, 128^3 with two poles 46 instead of 49), but not with two poles and x / y
+// layers (160 x 144 x 250 124 us with one cell, 141 with two); one with Kerr or the plasma
 // plug-ins (128 x 128 x 256 Kerr 108 instead of 113 us, 128 x 128 x 192 plasma
 // 109 instead of 116), with a design region (96^3 21.6 instead of 23.0) and in
 // FP64, whose two-cell form spills (192 x 192 x 384 551 instead of 691 us).
 template <typename T, int MODE, bool DESIGN, bool PLASMA>
-static cudaError_t launch_e_np(const EParams<T> &p, int np, cudaStream_t st) {
+static cudaError_t launch_e(const EParams<T> &p, int np, cudaStream_t st) {
   constexpr int V = sizeof(T) == 4 && MODE != MODE_PLRC_NONLIN && !DESIGN && !PLASMA ? 2 : 1;
-  return p.nx % V == 0 && p.nx > V ? launch_e_v<T, V, MODE, DESIGN, PLASMA>(p, np, st)
+  const bool two = p.nx % V == 0 && p.nx > V && !(np >= 2 && xy_faces(p));
+  return two ? launch_e_v<T, V, MODE, DESIGN, PLASMA>(p, np, st)
                                    : launch_e_v<T, 1, MODE, DESIGN, PLASMA>(p, np, st);
 }
 
@@ -565,24 +639,28 @@ cudaError_t launch_e_half(const EParams<T> &p, int mode, int np, cudaStream_t st
   const bool design = p.design.x0 <= p.design.x1;
   const bool plasma = p.rho != nullptr;
   switch (mode) {
-    case MODE_PLAIN: return launch_e_np<T, MODE_PLAIN, false, false>(p, 0, st);
-    case MODE_NL: return launch_e_np<T, MODE_NL, false, false>(p, 0, st);
+    case MODE_PLAIN: return launch_e<T, MODE_PLAIN, false, false>(p, 0, st);
+    case MODE_NL: return launch_e<T, MODE_NL, false, false>(p, 0, st);
     case MODE_PLRC_LIN:
-      return design   ? launch_e_np<T, MODE_PLRC_LIN, true, false>(p, np, st)
-             : plasma ? launch_e_np<T, MODE_PLRC_LIN, false, true>(p, np, st)
-                      : launch_e_np<T, MODE_PLRC_LIN, false, false>(p, np, st);
+      return design   ? launch_e<T, MODE_PLRC_LIN, true, false>(p, np, st)
+             : plasma ? launch_e<T, MODE_PLRC_LIN, false, true>(p, np, st)
+                      : launch_e<T, MODE_PLRC_LIN, false, false>(p, np, st);
     default:
-      return design   ? launch_e_np<T, MODE_PLRC_NONLIN, true, false>(p, np, st)
-             : plasma ? launch_e_np<T, MODE_PLRC_NONLIN, false, true>(p, np, st)
-                      : launch_e_np<T, MODE_PLRC_NONLIN, false, false>(p, np, st);
+      return design   ? launch_e<T, MODE_PLRC_NONLIN, true, false>(p, np, st)
+             : plasma ? launch_e<T, MODE_PLRC_NONLIN, false, true>(p, np, st)
+                      : launch_e<T, MODE_PLRC_NONLIN, false, false>(p, np, st);
   }
 }
 
 template <typename T, int V>
 static cudaError_t launch_b_v(const BParams<T> &p, cudaStream_t st) {
   dim3 d;
-  const RowGrid g = row_grid(p, V, max_planes<T>(), &d);
-  return launch_pdl(b_half_kernel<T, V>, d, dim3(kRowThreads, 1, 1), st, p, g);
+  const HalfGrid g = row_grid(p, V, max_planes<T>(), &d);
+  // early loads in FP32 only (FP64: 120 x 104 x 136 38 us either way, 192 x 192 x
+  // 384 220 instead of 200)
+  constexpr bool EARLY = sizeof(T) == 4;
+  return g.apart ? launch_pdl(b_half_kernel<T, V, EARLY>, d, dim3(kRowThreads, 1, 1), st, p, g)
+                 : launch_pdl(b_half_kernel<T, V, false>, d, dim3(kRowThreads, 1, 1), st, p, g);
 }
 
 // Two cells per thread in FP32 (256 x 256 x 512: 257 us, one cell 293, four
