@@ -32,54 +32,39 @@
 // The Kerr linearisation and the gradient accumulation are FP64; the rest is
 // in the precision of the forward state.  Latency-bound at small grids; one
 // thread per (x, y) column and chunk of planes.
-#include "mp_checked.cuh"
+#include "mp_cell.cuh"
 #include "mp_device.h"
 #include "mp_pdl.cuh"
+#include "mp_row.cuh"
+
+#include <algorithm>
 
 #include <cuda_runtime.h>
 
-// Blocks of 32 x MPB_ADJ_BLOCK_Y columns; resident threads per SM asked of
-// the register allocator, per precision.
-#ifndef MPB_ADJ_BLOCK_Y
-#define MPB_ADJ_BLOCK_Y 4
-#endif
-#ifndef MPB_ADJ_E_MIN_F
-#define MPB_ADJ_E_MIN_F 640
-#endif
-#ifndef MPB_ADJ_E_MIN_D
-#define MPB_ADJ_E_MIN_D 512
-#endif
-#ifndef MPB_ADJ_B_MIN_F
-#define MPB_ADJ_B_MIN_F 768
-#endif
-#ifndef MPB_ADJ_B_MIN_D
-#define MPB_ADJ_B_MIN_D 512
-#endif
-#define MPB_ADJ_THREADS (32 * MPB_ADJ_BLOCK_Y)
-
 namespace mpb {
+
+// Resident threads per SM asked of the register allocator: adj_e FP32 768 (512 /
+// 640 / 896 / 1024: the 96^3 reverse step 1.09 / 1.05 / 1.03 / 1.17 times as long),
+// FP64 512 (640: 216 instead of 180 us); adj_b FP32 1024, FP64 640 (512: 176
+// instead of 171 us, 120 x 104 x 136).
+template <typename T>
+__host__ __device__ constexpr int adj_e_threads() {
+  return sizeof(T) == 4 ? 768 : 512;
+}
+template <typename T>
+__host__ __device__ constexpr int adj_b_threads() {
+  return sizeof(T) == 4 ? 1024 : 640;
+}
 
 namespace {
 
-// Position of axis index idx in a face entry (-1: outside its layers).
+// Position of axis index idx in a face entry (-1: outside its layers; an entry
+// that is not active has empty layers).
 template <typename T>
 __device__ __forceinline__ int face_pos(const AdjFace<T> &F, int idx) {
-  if (!F.active) return -1;
   if (idx >= F.lo0 && idx <= F.hi0) return idx - F.lo0;
   if (idx >= F.lo1 && idx <= F.hi1) return F.n0 + idx - F.lo1;
   return -1;
-}
-
-// Element of the x (D = 0) or y (D = 1) entry at axis position pos, column
-// (i, j) and plane k: face_col(..) + face_plane(.., k).  32-bit: the host
-// keeps every face array below 2^31 elements.
-template <int D, typename T>
-__device__ __forceinline__ int face_col(const AdjFace<T> &F, int pos, int i, int j, int nx) {
-  return pos < 0 ? 0 : (D == 0 ? j * F.ex + pos : pos * nx + i);
-}
-template <int D, typename T>
-__device__ __forceinline__ int face_plane(const AdjFace<T> &F, int k, int nx, int ny) {
-  return D == 0 ? (k - F.zlo) * ny * F.ex : (k - F.zlo) * F.ey * nx;
 }
 
 // The components fed by psi0 / psi1 of a face along D (cpml_border.cpp:357-386):
@@ -93,106 +78,136 @@ __device__ __forceinline__ R comp1(const R v[3]) {
   return D == 0 ? v[2] : (D == 1 ? v[0] : v[1]);
 }
 
-// c * total at element li of an entry, or zero for pos < 0
-template <typename T, typename R>
-__device__ __forceinline__ void face_w(const AdjFace<T> &F, int pos, int li, R c, R &w0, R &w1, int *st) {
-  if (pos >= 0) {
-    w0 = c * R(ld_c(F.a0, li, F.n, st));
-    w1 = c * R(ld_c(F.a1, li, F.n, st));
-  } else {
-    w0 = w1 = R(0);
-  }
+// A thread's place in the x (D = 0) or y (D = 1) entry of a face pair: the
+// element of plane zlo, or -1 outside the layers.  32-bit: the host keeps every
+// face array below 2^31 elements.
+template <int D, typename T>
+__device__ __forceinline__ int face_at(const AdjFace<T> &F, int i, int j, int nx) {
+  const int pos = face_pos(F, D == 0 ? i + 1 : j + 1);
+  return pos < 0 ? -1 : (D == 0 ? j * F.ex + pos : pos * nx + i);
+}
+template <int D, typename T>
+__device__ __forceinline__ int face_plane(const AdjFace<T> &F, int k, int nx, int ny) {
+  return D == 0 ? (k - F.zlo) * ny * F.ex : (k - F.zlo) * F.ey * nx;
+}
+
+// c * total of both components at element li of an entry
+template <typename T>
+__device__ __forceinline__ void face_w(const AdjFace<T> &F, int li, T c, T &w0, T &w1, int *st) {
+  w0 = c * ld_c(F.a0, li, F.n, st);
+  w1 = c * ld_c(F.a1, li, F.n, st);
+}
+
+// One element of column c of the plane at element `base` (a uniform address
+// plus a 32-bit offset, as ldp / stp).
+template <typename T>
+__device__ __forceinline__ T at(const T *a, long long base, unsigned c, long long n, int *st) {
+  return ldp<1>(a, base, c, n, st).v[0];
+}
+template <typename T>
+__device__ __forceinline__ void put(T *a, long long base, unsigned c, long long n, int *st, T v) {
+  RowV<T, 1> r;
+  r.v[0] = v;
+  stp<1>(a, base, c, n, st, r);
+}
+
+// The new total of an entry: b * total + dt * what it feeds
+template <typename T>
+__device__ __forceinline__ void face_step(const AdjFace<T> &F, int li, T b, T t0, T t1, T dt, T f0, T f1, int *st) {
+  st_c(F.a0, li, F.n, st, T(b * t0 + dt * f0));
+  st_c(F.a1, li, F.n, st, T(b * t1 + dt * f1));
 }
 
 }  // namespace
 
+// The z-chunks of the reverse kernels over the row mapping of mp_row.cuh, and
+// the planes whose z faces hold something: k <= zlo or k >= zhi.
+struct AdjGrid : RowMap {
+  int kchunk, zlo, zhi;
+  int ahead;  // prefetch the next plane into L2
+};
+
 // Arithmetic is in T (the precision of the state); the Kerr linearisation and
 // the design gradients are FP64.  One thread per (x, y) column marches up a
-// chunk of planes, carrying the z-neighbours in registers.  Arrays a kernel
-// only reads (the B adjoint in adj_e, G in adj_b, the E history) go through
-// the read-only data path (ldg_c).  NL: the Kerr medium (PLRC nonlinear); the
-// linear form leaves out the Kerr linearisation, whose terms are zero there.
+// chunk of planes, carrying the z-neighbours in registers; the cells are dealt
+// to threads as in the half steps (row_cells).  NL: the Kerr medium (PLRC
+// nonlinear); the linear form leaves out the Kerr linearisation, whose terms are
+// zero there.
+// A thread finds its place in the x and y face entries once, before the march,
+// and a plane tests three flags: its columns lie in an x entry, in a y entry, the
+// plane in a z entry.  On grids that exceed L2 bound by HBM and its latency (the
+// next plane is prefetched into L2), on smaller ones by instruction issue (96^3
+// with CPML on all faces: 60% of the issue slots).  Reverse step (adj_e + adj_b),
+// before -> after: 96^3 FP32 43.6 -> 40.0 us, 120 x 104 x 136 FP64 Kerr 207 -> 162,
+// 160 x 144 x 160 FP32 Kerr 229 -> 185, 256^3 FP32 Kerr 1100 -> 778, 192 x 192 x
+// 256 FP64 774 -> 546.
 template <typename T, int NP, bool NL>
-__global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_MIN_F : MPB_ADJ_E_MIN_D) / MPB_ADJ_THREADS)
-    adj_e_kernel(const AdjParams<T> p) {
+__global__ void __launch_bounds__(kRowThreads, adj_e_threads<T>() / kRowThreads)
+    adj_e_kernel(const AdjParams<T> p, const AdjGrid g) {
   typedef T R;
+  typedef typename Vec2<T>::type T2;
   pdl_launch_dependents();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= p.nx || j >= p.ny) return;
-  const int k0 = 1 + blockIdx.z * p.kchunk_e;
-  const int k1 = min(k0 + p.kchunk_e - 1, p.nz);
-  if (k0 > k1) return;
   const int nx = p.nx, ny = p.ny;
+  int i, j;
+  if (!row_cells<1>(g, blockIdx.x, ny, i, j)) return;
+  const int k0 = 1 + blockIdx.y * g.kchunk;
+  const int k1 = min(k0 + g.kchunk - 1, p.nz);
   const int im = i == 0 ? nx - 1 : i - 1;
   const int jm = j == 0 ? ny - 1 : j - 1;
   const long long pl = p.plane;
-  const int col = j * nx + i, colxm = j * nx + im, colym = jm * nx + i;
+  const unsigned row = unsigned(j) * unsigned(nx);
+  const unsigned col = row + i, colxm = row + im, colym = unsigned(jm) * unsigned(nx) + i;
   const R dt = R(p.dt);
   const long long nf = p.n_field;
   int *const st = p.status;
-  const R kxi = p.ikH[0][i + 1], kxm = p.ikH[0][im + 1];
-  const R kyj = p.ikH[1][j + 1], kym = p.ikH[1][jm + 1];
-  const R bzj = p.ikH_bzy[j + 1], bzm = p.ikH_bzy[jm + 1];
+  const R kxi = ld(p.ikH[0] + i + 1), kxm = ld(p.ikH[0] + im + 1);
+  const R kyj = ld(p.ikH[1] + j + 1), kym = ld(p.ikH[1] + jm + 1);
+  const R bzj = ld(p.ikH_bzy + j + 1), bzm = ld(p.ikH_bzy + jm + 1);
   const T *Bx = p.Bb[0], *By = p.Bb[1], *Bz = p.Bb[2];
   const AdjFace<T> &HX = p.fh[0], &HY = p.fh[1], &HZ = p.fh[2];
   const AdjFace<T> &EX = p.fe[0], &EY = p.fe[1], &EZ = p.fe[2];
-  const int plane = int(pl);
-  // warps whose columns lie in no x / y face skip the face code on planes
-  // outside the z faces; the face positions are recomputed where used
-  const bool warp_xy = __any_sync(__activemask(), (face_pos(HX, i + 1) >= 0) || (face_pos(HX, im + 1) >= 0) ||
-                                                      (face_pos(HY, j + 1) >= 0) || (face_pos(HY, jm + 1) >= 0) ||
-                                                      (face_pos(EX, i + 1) >= 0) || (face_pos(EY, j + 1) >= 0));
-  // everything below reads what the previous reverse kernel wrote
-  pdl_wait();
-  // the z H face's c * total at plane k - 1, carried
-  R cw0, cw1;
-  bool cw_on;
-  {
-    const int pz = face_pos(HZ, k0 - 1);
-    cw_on = pz >= 0;
-    face_w(HZ, pz, pz * plane + col, pz >= 0 ? R(HZ.c[k0 - 1]) : R(0), cw0, cw1, st);
-  }
+  // this column (o) and its x-1 / y-1 neighbour (m) in the face entries
+  const int hxo = face_at<0>(HX, i, j, nx), hxm = face_at<0>(HX, im, j, nx), exo = face_at<0>(EX, i, j, nx);
+  const int hyo = face_at<1>(HY, i, j, nx), hym = face_at<1>(HY, i, jm, nx), eyo = face_at<1>(EY, i, j, nx);
+  const bool fx = (hxo & hxm & exo) != -1, fy = (hyo & hym & eyo) != -1;
   const DesignParams &d = p.design;
   const bool dxy = i >= d.x0 && i <= d.x1 && j >= d.y0 && j <= d.y1;
-  const bool oxy = i >= p.ox0 && i <= p.ox1 && j >= p.oy0 && j <= p.oy1;
-  R bx_km = ldg_c(Bx, (long long)(k0 - 1) * pl + col, nf, st);
-  R by_km = ldg_c(By, (long long)(k0 - 1) * pl + col, nf, st);
+  const bool oxy = p.add_obj && i >= p.ox0 && i <= p.ox1 && j >= p.oy0 && j <= p.oy1;
+  // everything below reads what the previous reverse kernel wrote
+  pdl_wait();
+  R bx_km = at(Bx, (k0 - 1) * pl, col, nf, st);
+  R by_km = at(By, (k0 - 1) * pl, col, nf, st);
 
-  const bool plrc_nl = NL;
   for (int k = k0; k <= k1; ++k) {
     const long long base = (long long)k * pl;
-    const long long c0 = base + col;
     const bool med = k >= p.mz0 && k <= p.mz1;
     const bool dcell = med && dxy && k >= d.z0 && k <= d.z1;
     // ---- every load of this plane first, so that their latencies overlap
-    const R bx = ldg_c(Bx, c0, nf, st), by = ldg_c(By, c0, nf, st), bz = ldg_c(Bz, c0, nf, st);
-    const R bx_ym = ldg_c(Bx, base + colym, nf, st), by_xm = ldg_c(By, base + colxm, nf, st),
-            bz_ym = ldg_c(Bz, base + colym, nf, st), bz_xm = ldg_c(Bz, base + colxm, nf, st);
-    const R kzk = p.ikH[2][k], kzm = p.ikH[2][k - 1];
-    R a[3] = {R(ld_c(p.Eb[0], c0, nf, st)), R(ld_c(p.Eb[1], c0, nf, st)), R(ld_c(p.Eb[2], c0, nf, st))};
+    const R bx = at(Bx, base, col, nf, st), by = at(By, base, col, nf, st), bz = at(Bz, base, col, nf, st);
+    const R bx_ym = at(Bx, base, colym, nf, st), by_xm = at(By, base, colxm, nf, st),
+            bz_ym = at(Bz, base, colym, nf, st), bz_xm = at(Bz, base, colxm, nf, st);
+    const R kzk = ld(p.ikH[2] + k), kzm = ld(p.ikH[2] + k - 1);
+    R a[3] = {at(p.Eb[0], base, col, nf, st), at(p.Eb[1], base, col, nf, st), at(p.Eb[2], base, col, nf, st)};
     // E^n enters here only through the Kerr term (its coefficient is zero in
     // a linear medium) and the |E|^2 objective's box: elsewhere it is not read
     R En[3] = {R(0), R(0), R(0)};
-    if (plrc_nl || (p.add_obj && oxy && p.obj_kind == 1 && k >= p.oz0 && k <= p.oz1)) {
+    if (NL || (oxy && p.obj_kind == 1 && k >= p.oz0 && k <= p.oz1)) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) En[c] = R(ldg_c(p.En[c], c0, nf, st));
+      for (int c = 0; c < 3; ++c) En[c] = at(p.En[c], base, col, nf, st);
     }
     R En1[3] = {R(0), R(0), R(0)};
-    if (med && (plrc_nl || dcell)) {
+    if (NL && med) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) En1[c] = R(ldg_c(p.En1[c], c0, nf, st));
+      for (int c = 0; c < 3; ++c) En1[c] = at(p.En1[c], base, col, nf, st);
     }
-    const long long pi = ((long long)(k - p.mz0) * ny + j) * nx + i;
-    R pq[NP > 0 ? NP : 1][3][2];
-    if (med) {
+    const long long pbase = (long long)(k - p.mz0) * pl;
+    T2 pq[NP > 0 ? NP : 1][3];
+    if (NP > 0 && med) {
 #pragma unroll
       for (int n = 0; n < NP; ++n)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          pq[n][c][0] = ld_c(p.psib[n][c], 2 * pi, 2 * p.n_psi, st);
-          pq[n][c][1] = ld_c(p.psib[n][c], 2 * pi + 1, 2 * p.n_psi, st);
-        }
+        for (int c = 0; c < 3; ++c)
+          pq[n][c] = at(reinterpret_cast<const T2 *>(p.psib[n][c]), pbase, col, p.n_psi, st);
     }
     long long di = 0;
     double e = p.eps, s = 1.0, u = 1.0;
@@ -202,38 +217,53 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
       s = ld_c(d.dscale, di, p.n_design, st);
       u = ld_c(d.chiscale, di, p.n_design, st);
     }
-    // H-face totals (x, y at this column and x-1 / y-1; z at this plane) and
-    // E-face totals of this cell, on warps and planes that touch a face
-    const int hzp = face_pos(HZ, k), ezp = face_pos(EZ, k);
-    const bool fpl = warp_xy || cw_on || hzp >= 0 || ezp >= 0;
+    if (g.ahead && k < k1) {
+      const long long bn = base + pl;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        prefetch_l2(p.Bb[c] + bn + col);
+        prefetch_l2(p.Eb[c] + bn + col);
+        if (NL) prefetch_l2(p.En[c] + bn + col);
+        if (NL) prefetch_l2(p.En1[c] + bn + col);
+        if (med) {
+#pragma unroll
+          for (int n = 0; n < NP; ++n)
+            prefetch_l2(reinterpret_cast<const T2 *>(p.psib[n][c]) + pbase + pl + col);
+        }
+      }
+    }
+    // H-face totals (at this column and x-1 / y-1, at this plane and k-1) and
+    // E-face totals of this cell
+    const bool fz = k <= g.zlo || k >= g.zhi;
     R hx0o = R(0), hx1o = R(0), hx0m = R(0), hx1m = R(0), hy0o = R(0), hy1o = R(0), hy0m = R(0), hy1m = R(0);
-    R hz0 = R(0), hz1 = R(0);
-    R ex0 = R(0), ex1 = R(0), ey0 = R(0), ey1 = R(0), ez0 = R(0), ez1 = R(0), ezb = R(0);
-    int lexo = 0, leyo = 0, lezo = 0;
-    if (fpl) {
-      const int hxo = face_pos(HX, i + 1), hxm = face_pos(HX, im + 1);
-      const int hyo = face_pos(HY, j + 1), hym = face_pos(HY, jm + 1);
-      const R hxco = hxo >= 0 ? R(HX.c[i + 1]) : R(0), hxcm = hxm >= 0 ? R(HX.c[im + 1]) : R(0);
-      const R hyco = hyo >= 0 ? R(HY.c[j + 1]) : R(0), hycm = hym >= 0 ? R(HY.c[jm + 1]) : R(0);
-      const int exo = face_pos(EX, i + 1), eyo = face_pos(EY, j + 1);
-      const int chxo = face_col<0>(HX, hxo, i, j, nx), chxm = face_col<0>(HX, hxm, im, j, nx);
-      const int chyo = face_col<1>(HY, hyo, i, j, nx), chym = face_col<1>(HY, hym, i, jm, nx);
-      const int cexo = face_col<0>(EX, exo, i, j, nx), ceyo = face_col<1>(EY, eyo, i, j, nx);
-      const int shx = face_plane<0>(HX, k, nx, ny), shy = face_plane<1>(HY, k, nx, ny);
-      face_w(HX, hxo, chxo + shx, hxco, hx0o, hx1o, st);
-      face_w(HX, hxm, chxm + shx, hxcm, hx0m, hx1m, st);
-      face_w(HY, hyo, chyo + shy, hyco, hy0o, hy1o, st);
-      face_w(HY, hym, chym + shy, hycm, hy0m, hy1m, st);
-      face_w(HZ, hzp, hzp * plane + col, hzp >= 0 ? R(HZ.c[k]) : R(0), hz0, hz1, st);
-      lexo = exo >= 0 ? cexo + face_plane<0>(EX, k, nx, ny) : -1;
-      leyo = eyo >= 0 ? ceyo + face_plane<1>(EY, k, nx, ny) : -1;
-      lezo = ezp * plane + col;
-      if (lexo >= 0) { ex0 = ld_c(EX.a0, lexo, EX.n, st); ex1 = ld_c(EX.a1, lexo, EX.n, st); }
-      if (leyo >= 0) { ey0 = ld_c(EY.a0, leyo, EY.n, st); ey1 = ld_c(EY.a1, leyo, EY.n, st); }
-      if (ezp >= 0) { ez0 = ld_c(EZ.a0, lezo, EZ.n, st); ez1 = ld_c(EZ.a1, lezo, EZ.n, st); ezb = EZ.b[k]; }
+    R hz0 = R(0), hz1 = R(0), cw0 = R(0), cw1 = R(0);
+    R ex0 = R(0), ex1 = R(0), ey0 = R(0), ey1 = R(0), ez0 = R(0), ez1 = R(0);
+    int lex = 0, ley = 0, lez = 0, ezp = -1;
+    if (fx) {
+      const int sh = face_plane<0>(HX, k, nx, ny);
+      if (hxo >= 0) face_w(HX, hxo + sh, ld(HX.c + i + 1), hx0o, hx1o, st);
+      if (hxm >= 0) face_w(HX, hxm + sh, ld(HX.c + im + 1), hx0m, hx1m, st);
+      lex = exo + face_plane<0>(EX, k, nx, ny);
+      if (exo >= 0) face_w(EX, lex, R(1), ex0, ex1, st);
+    }
+    if (fy) {
+      const int sh = face_plane<1>(HY, k, nx, ny);
+      if (hyo >= 0) face_w(HY, hyo + sh, ld(HY.c + j + 1), hy0o, hy1o, st);
+      if (hym >= 0) face_w(HY, hym + sh, ld(HY.c + jm + 1), hy0m, hy1m, st);
+      ley = eyo + face_plane<1>(EY, k, nx, ny);
+      if (eyo >= 0) face_w(EY, ley, R(1), ey0, ey1, st);
+    }
+    if (fz) {
+      const int hzp = face_pos(HZ, k), hzm = face_pos(HZ, k - 1);
+      if (hzp >= 0) face_w(HZ, hzp * int(pl) + int(col), ld(HZ.c + k), hz0, hz1, st);
+      if (hzm >= 0) face_w(HZ, hzm * int(pl) + int(col), ld(HZ.c + k - 1), cw0, cw1, st);
+      ezp = face_pos(EZ, k);
+      lez = ezp * int(pl) + int(col);
+      if (ezp >= 0) face_w(EZ, lez, R(1), ez0, ez1, st);
     }
     R obx = R(0), oby = R(0);
-    if (p.add_obj && oxy && p.obj_kind == 2 && k == p.oz0) {
+    const bool osz = oxy && p.obj_kind == 2 && k == p.oz0;
+    if (osz) {
       obx = ld_c(p.obx, col, pl, st);
       oby = ld_c(p.oby, col, pl, st);
     }
@@ -250,26 +280,27 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
     a[1] += dt * (-kxm * bz_xm + kxi * bz);
     // H faces: psi0 / psi1 feed (y, z) on x faces, (z, x) on y faces, (x, y) on
     // z faces; their differences of E run forward along the axis
-    if (fpl) {
+    if (fx) {
       a[2] += hx0m - hx0o;
       a[1] += hx1o - hx1m;
+    }
+    if (fy) {
       a[0] += hy0m - hy0o;
       a[2] += hy1o - hy1m;
+    }
+    if (fz) {
       a[1] += cw0 - hz0;
       a[0] += hz1 - cw1;
     }
-    cw0 = hz0;
-    cw1 = hz1;
-    cw_on = hzp >= 0;
 
     // ---- E half, locally
-    R g[3], ne[3];
+    R gg[3], ne[3];
     if (!med) {
       // background: E' = (eps_bg E + dt (curl + J)) / eps_bg
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        g[c] = a[c] * p.inv_eps_bg_t;
-        ne[c] = p.eps_bg_t * g[c];
+        gg[c] = a[c] * p.inv_eps_bg_t;
+        ne[c] = p.eps_bg_t * gg[c];
       }
     } else {
       double A = NL ? p.A0 : 0.0;
@@ -284,11 +315,12 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
       R cb[3] = {a[0], a[1], a[2]};
       if (NL) {
         // E' = r c/|c| with r + A r^3 = |c|: dE'/dc = (I - e e^T) / (1 + A r^2)
-        // + e e^T / (1 + 3 A r^2), dr/dA = -r^3 / (1 + 3 A r^2), c = E' (1 + A r^2)
-        const double r2 = (double)En1[0] * En1[0] + (double)En1[1] * En1[1] + (double)En1[2] * En1[2];
-        const double r = sqrt(r2);
-        const double al = 1.0 / (1.0 + A * r2), be = 1.0 / (1.0 + 3.0 * A * r2);
-        const double ir = r > 0 ? 1.0 / r : 0.0;
+        // + e e^T / (1 + 3 A r^2), dr/dA = -r^3 / (1 + 3 A r^2), c = E' (1 + A r^2);
+        // the reciprocals of the denominators (>= 1) and of r as in the forward
+        // Kerr update (FP64, exact to rounding)
+        const double r2 = sq3((double)En1[0], (double)En1[1], (double)En1[2]);
+        const double al = rcp_pos(1.0 + A * r2), be = rcp_pos(1.0 + 3.0 * A * r2);
+        const double ir = r2 > 0 ? rsqrt(r2) : 0.0;
         double eh[3], ea = 0.0;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -299,16 +331,16 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
         for (int c = 0; c < 3; ++c) cb[c] = R(al * (a[c] - eh[c] * ea) + be * eh[c] * ea);
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) g[c] = cb[c] * idn;
+      for (int c = 0; c < 3; ++c) gg[c] = cb[c] * idn;
       if (NL) {
         const R E2 = En[0] * En[0] + En[1] * En[1] + En[2] * En[2];
-        const R Eg = En[0] * g[0] + En[1] * g[1] + En[2] * g[2];
+        const R Eg = En[0] * gg[0] + En[1] * gg[1] + En[2] * gg[2];
         const R f = numer + Rchi * E2;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) ne[c] = f * g[c] + R(2) * Rchi * En[c] * Eg;
+        for (int c = 0; c < 3; ++c) ne[c] = f * gg[c] + R(2) * Rchi * En[c] * Eg;
       } else {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) ne[c] = numer * g[c];
+        for (int c = 0; c < 3; ++c) ne[c] = numer * gg[c];
       }
       // the design cells' accumulator adjoints before the reverse recursion,
       // for adj_grad
@@ -316,11 +348,8 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
 #pragma unroll
         for (int n = 0; n < NP; ++n)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const long long q = ((di * NP + n) * 3 + c) * 2;
-            st_c(p.dpsi, q, p.n_design * NP * 6, st, T(pq[n][c][0]));
-            st_c(p.dpsi, q + 1, p.n_design * NP * 6, st, T(pq[n][c][1]));
-          }
+          for (int c = 0; c < 3; ++c)
+            st_c(reinterpret_cast<T2 *>(p.dpsi), (di * NP + n) * 3 + c, p.n_design * NP * 3, st, pq[n][c]);
       }
       // reverse PLRC recursion: psi~bar = conj(Crec) psibar + g
       const R Rs = dcell ? R(s) : R(1);
@@ -331,60 +360,41 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
         const R Cr = p.pCt[n][0], Ci = p.pCt[n][1];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const R pr = pq[n][c][0], pim = pq[n][c][1];
-          const R tr = Cr * pr + Ci * pim + g[c];
+          const R pr = pq[n][c].x, pim = pq[n][c].y;
+          const R tr = Cr * pr + Ci * pim + gg[c];
           const R ti = Cr * pim - Ci * pr;
           ne[c] += Rs * (Dr * tr + Di * ti + Xr * pr + Xi * pim);
-          pq[n][c][0] = tr;
-          pq[n][c][1] = ti;
+          pq[n][c].x = tr;
+          pq[n][c].y = ti;
         }
       }
     }
     // the objective's E term of the state before the step
-    if (p.add_obj && oxy) {
-      if (p.obj_kind == 1) {
-        if (k >= p.oz0 && k <= p.oz1) {
+    if (oxy && p.obj_kind == 1 && k >= p.oz0 && k <= p.oz1) {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) ne[c] += p.obj_f_t * En[c];
-        }
-      } else if (k == p.oz0) {
-        ne[0] += p.obj_f_t * oby;
-        ne[1] -= p.obj_f_t * obx;
-      }
+      for (int c = 0; c < 3; ++c) ne[c] += p.obj_f_t * En[c];
+    }
+    if (osz) {
+      ne[0] += p.obj_f_t * oby;
+      ne[1] -= p.obj_f_t * obx;
     }
 
     // ---- stores
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      st_c(p.G[c], c0, nf, st, T(g[c]));
-      st_c(p.Eb[c], c0, nf, st, T(ne[c]));
+      put(p.G[c], base, col, nf, st, gg[c]);
+      put(p.Eb[c], base, col, nf, st, ne[c]);
     }
-    if (med) {
+    if (NP > 0 && med) {
 #pragma unroll
       for (int n = 0; n < NP; ++n)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          st_c(p.psib[n][c], 2 * pi, 2 * p.n_psi, st, T(pq[n][c][0]));
-          st_c(p.psib[n][c], 2 * pi + 1, 2 * p.n_psi, st, T(pq[n][c][1]));
-        }
+        for (int c = 0; c < 3; ++c) put(reinterpret_cast<T2 *>(p.psib[n][c]), pbase, col, p.n_psi, st, pq[n][c]);
     }
     // E-face totals of this cell: b * total + dt * G
-    if (fpl) {
-      if (lexo >= 0) {
-        const R exb = R(EX.b[i + 1]);
-        st_c(EX.a0, lexo, EX.n, st, T(exb * ex0 + dt * comp0<0>(g)));
-        st_c(EX.a1, lexo, EX.n, st, T(exb * ex1 + dt * comp1<0>(g)));
-      }
-      if (leyo >= 0) {
-        const R eyb = R(EY.b[j + 1]);
-        st_c(EY.a0, leyo, EY.n, st, T(eyb * ey0 + dt * comp0<1>(g)));
-        st_c(EY.a1, leyo, EY.n, st, T(eyb * ey1 + dt * comp1<1>(g)));
-      }
-      if (ezp >= 0) {
-        st_c(EZ.a0, lezo, EZ.n, st, T(ezb * ez0 + dt * comp0<2>(g)));
-        st_c(EZ.a1, lezo, EZ.n, st, T(ezb * ez1 + dt * comp1<2>(g)));
-      }
-    }
+    if (fx && exo >= 0) face_step(EX, lex, ld(EX.b + i + 1), ex0, ex1, dt, comp0<0>(gg), comp1<0>(gg), st);
+    if (fy && eyo >= 0) face_step(EY, ley, ld(EY.b + j + 1), ey0, ey1, dt, comp0<1>(gg), comp1<1>(gg), st);
+    if (fz && ezp >= 0) face_step(EZ, lez, ld(EZ.b + k), ez0, ez1, dt, comp0<2>(gg), comp1<2>(gg), st);
     bx_km = bx;
     by_km = by;
   }
@@ -407,7 +417,7 @@ __global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_E_M
 template <typename T, int NP, bool NL>
 __device__ __forceinline__ void adj_grad_cells(const AdjParams<T> &p, int gbx, int gby, int kk) {
   const DesignParams &d = p.design;
-  const int ii = gbx * blockDim.x + threadIdx.x, jj = gby * blockDim.y + threadIdx.y;
+  const int ii = gbx * 32 + (threadIdx.x & 31), jj = gby * kRowTile + (threadIdx.x >> 5);
   if (ii >= d.bx || jj >= d.by) return;
   pdl_wait();
   const int i = d.x0 + ii, j = d.y0 + jj, k = d.z0 + kk;
@@ -421,8 +431,8 @@ __device__ __forceinline__ void adj_grad_cells(const AdjParams<T> &p, int gbx, i
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     g[c] = ld_c(p.G[c], c0, nf, st);
-    En[c] = ldg_c(p.En[c], c0, nf, st);
-    En1[c] = ldg_c(p.En1[c], c0, nf, st);
+    En[c] = ld_c(p.En[c], c0, nf, st);
+    En1[c] = ld_c(p.En1[c], c0, nf, st);
   }
   const double dD = p.sumChi0 - p.sumXi0;
   const double denom = d.lin ? e + s * dD : e + s * p.sumChi0 - s * p.sumXi0;
@@ -470,95 +480,91 @@ __device__ __forceinline__ void adj_grad_cells(const AdjParams<T> &p, int gbx, i
 }
 
 template <typename T>
-__device__ __forceinline__ void adj_b_cells(const AdjParams<T> &p, int bxi, int byi, int bzi) {
+__device__ __forceinline__ void adj_b_cells(const AdjParams<T> &p, const AdjGrid &g, unsigned block, int chunk) {
   typedef T R;
-  const int i = bxi * blockDim.x + threadIdx.x;
-  const int j = byi * blockDim.y + threadIdx.y;
-  if (i >= p.nx || j >= p.ny) return;
-  const int k0 = bzi * p.kchunk_b;
-  const int k1 = min(k0 + p.kchunk_b - 1, p.nz);
-  if (k0 > k1) return;
   const int nx = p.nx, ny = p.ny;
+  int i, j;
+  if (!row_cells<1>(g, block, ny, i, j)) return;
+  const int k0 = chunk * g.kchunk;
+  const int k1 = min(k0 + g.kchunk - 1, p.nz);
   const int ip = i == nx - 1 ? 0 : i + 1;
   const int jp = j == ny - 1 ? 0 : j + 1;
   const long long pl = p.plane;
-  const int col = j * nx + i, colxp = j * nx + ip, colyp = jp * nx + i;
+  const unsigned row = unsigned(j) * unsigned(nx);
+  const unsigned col = row + i, colxp = row + ip, colyp = unsigned(jp) * unsigned(nx) + i;
   const R dt = R(p.dt);
   const long long nf = p.n_field;
   int *const st = p.status;
-  const R kxi = p.ikE[0][i + 1], kxp = p.ikE[0][ip + 1];
-  const R kyj = p.ikE[1][j + 1], kyp = p.ikE[1][jp + 1];
+  const R kxi = ld(p.ikE[0] + i + 1), kxp = ld(p.ikE[0] + ip + 1);
+  const R kyj = ld(p.ikE[1] + j + 1), kyp = ld(p.ikE[1] + jp + 1);
   const T *gx = p.G[0], *gy = p.G[1], *gz = p.G[2];
   const AdjFace<T> &HX = p.fh[0], &HY = p.fh[1], &HZ = p.fh[2];
   const AdjFace<T> &EX = p.fe[0], &EY = p.fe[1], &EZ = p.fe[2];
-  // E faces at this column and at x+1 / y+1; H faces at this column
-  const int exo = face_pos(EX, i + 1), exp_ = face_pos(EX, ip + 1);
-  const int eyo = face_pos(EY, j + 1), eyp = face_pos(EY, jp + 1);
-  const R exco = exo >= 0 ? R(EX.c[i + 1]) : R(0), excp = exp_ >= 0 ? R(EX.c[ip + 1]) : R(0);
-  const R eyco = eyo >= 0 ? R(EY.c[j + 1]) : R(0), eycp = eyp >= 0 ? R(EY.c[jp + 1]) : R(0);
-  const int hxo = face_pos(HX, i + 1), hyo = face_pos(HY, j + 1);
-  const R hxb = hxo >= 0 ? R(HX.b[i + 1]) : R(0), hyb = hyo >= 0 ? R(HY.b[j + 1]) : R(0);
+  // this column (o) and its x+1 / y+1 neighbour (p) in the face entries
+  const int exo = face_at<0>(EX, i, j, nx), exp_ = face_at<0>(EX, ip, j, nx), hxo = face_at<0>(HX, i, j, nx);
+  const int eyo = face_at<1>(EY, i, j, nx), eyp = face_at<1>(EY, i, jp, nx), hyo = face_at<1>(HY, i, j, nx);
+  const bool fx = (exo & exp_ & hxo) != -1, fy = (eyo & eyp & hyo) != -1;
   const bool oxy = p.add_obj && p.obj_kind == 2 && i >= p.ox0 && i <= p.ox1 && j >= p.oy0 && j <= p.oy1;
-  const int plane = int(pl);
-  const int cexo = face_col<0>(EX, exo, i, j, nx), cexp = face_col<0>(EX, exp_, ip, j, nx);
-  const int ceyo = face_col<1>(EY, eyo, i, j, nx), ceyp = face_col<1>(EY, eyp, i, jp, nx);
-  const int chxo = face_col<0>(HX, hxo, i, j, nx), chyo = face_col<1>(HY, hyo, i, j, nx);
-  // warps whose columns lie in no x / y face skip the face code on planes
-  // outside the z faces
-  const bool warp_xy =
-      __any_sync(__activemask(), (exo >= 0) || (exp_ >= 0) || (eyo >= 0) || (eyp >= 0) || (hxo >= 0) || (hyo >= 0));
   // everything below reads what adj_e wrote
   pdl_wait();
-  // G and the z E face's c * total at plane k, carried from the previous plane's k + 1
-  R gx_k = ldg_c(gx, (long long)k0 * pl + col, nf, st), gy_k = ldg_c(gy, (long long)k0 * pl + col, nf, st);
-  R zw0, zw1;
-  bool zw_on;
-  {
-    const int pz = face_pos(EZ, k0);
-    zw_on = pz >= 0;
-    face_w(EZ, pz, pz * plane + col, pz >= 0 ? R(EZ.c[k0]) : R(0), zw0, zw1, st);
-  }
+  // G at plane k, carried from the previous plane's k + 1
+  R gx_k = at(gx, k0 * pl, col, nf, st), gy_k = at(gy, k0 * pl, col, nf, st);
 
   for (int k = k0; k <= k1; ++k) {
     const long long base = (long long)k * pl;
-    const long long c0 = base + col;
     // ---- every load of this plane first
-    const R gx_kp = ldg_c(gx, c0 + pl, nf, st), gy_kp = ldg_c(gy, c0 + pl, nf, st);
-    const R gzk = ldg_c(gz, c0, nf, st);
-    const R gx_yp = ldg_c(gx, base + colyp, nf, st), gy_xp = ldg_c(gy, base + colxp, nf, st),
-            gz_xp = ldg_c(gz, base + colxp, nf, st), gz_yp = ldg_c(gz, base + colyp, nf, st);
-    const R kzk = p.ikE[2][k], kzp = p.ikE[2][k + 1];
-    R b[3] = {R(ld_c(p.Bb[0], c0, nf, st)), R(ld_c(p.Bb[1], c0, nf, st)), R(ld_c(p.Bb[2], c0, nf, st))};
-    // faces on warps and planes that touch one: E faces (x / y hold planes
-    // 1..nz; z at plane k + 1, plane k carried) and the H-face totals of this cell
-    const int ezq = face_pos(EZ, k + 1), hzp = face_pos(HZ, k);
-    const bool fpl = warp_xy || zw_on || ezq >= 0 || hzp >= 0;
+    const R gx_kp = at(gx, base + pl, col, nf, st), gy_kp = at(gy, base + pl, col, nf, st);
+    const R gzk = at(gz, base, col, nf, st);
+    const R gx_yp = at(gx, base, colyp, nf, st), gy_xp = at(gy, base, colxp, nf, st),
+            gz_xp = at(gz, base, colxp, nf, st), gz_yp = at(gz, base, colyp, nf, st);
+    const R kzk = ld(p.ikE[2] + k), kzp = ld(p.ikE[2] + k + 1);
+    R b[3] = {at(p.Bb[0], base, col, nf, st), at(p.Bb[1], base, col, nf, st), at(p.Bb[2], base, col, nf, st)};
+    if (g.ahead && k < k1) {
+      const long long bn = base + pl;
+      prefetch_l2(gx + bn + pl + col);
+      prefetch_l2(gy + bn + pl + col);
+      prefetch_l2(gz + bn + col);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) prefetch_l2(p.Bb[c] + bn + col);
+    }
+    // E faces (x / y hold planes 1..nz; z at planes k and k + 1) and the
+    // H-face totals of this cell
+    const bool fz = k <= g.zlo || k >= g.zhi;
     R ex0o = R(0), ex1o = R(0), ex0p = R(0), ex1p = R(0), ey0o = R(0), ey1o = R(0), ey0p = R(0), ey1p = R(0);
-    R ez0p = R(0), ez1p = R(0);
-    const bool hxk = hxo >= 0 && k >= HX.zlo, hyk = hyo >= 0 && k >= HY.zlo;
-    int lhx = 0, lhy = 0, lhz = 0;
-    R hx0 = R(0), hx1 = R(0), hy0 = R(0), hy1 = R(0), hz0 = R(0), hz1 = R(0), hzb = R(0);
-    if (fpl) {
-      if (k >= 1) {
-        const int sex = face_plane<0>(EX, k, nx, ny), sey = face_plane<1>(EY, k, nx, ny);
-        face_w(EX, exo, cexo + sex, exco, ex0o, ex1o, st);
-        face_w(EX, exp_, cexp + sex, excp, ex0p, ex1p, st);
-        face_w(EY, eyo, ceyo + sey, eyco, ey0o, ey1o, st);
-        face_w(EY, eyp, ceyp + sey, eycp, ey0p, ey1p, st);
+    R zw0 = R(0), zw1 = R(0), ez0p = R(0), ez1p = R(0);
+    R hx0 = R(0), hx1 = R(0), hy0 = R(0), hy1 = R(0), hz0 = R(0), hz1 = R(0);
+    int lhx = -1, lhy = -1, lhz = 0, hzp = -1;
+    if (fx) {
+      const int se = face_plane<0>(EX, k, nx, ny);
+      if (exo >= 0 && k >= 1) face_w(EX, exo + se, ld(EX.c + i + 1), ex0o, ex1o, st);
+      if (exp_ >= 0 && k >= 1) face_w(EX, exp_ + se, ld(EX.c + ip + 1), ex0p, ex1p, st);
+      if (hxo >= 0 && k >= HX.zlo) {
+        lhx = hxo + face_plane<0>(HX, k, nx, ny);
+        face_w(HX, lhx, R(1), hx0, hx1, st);
       }
-      face_w(EZ, ezq, ezq * plane + col, ezq >= 0 ? R(EZ.c[k + 1]) : R(0), ez0p, ez1p, st);
-      lhx = chxo + face_plane<0>(HX, k, nx, ny);
-      lhy = chyo + face_plane<1>(HY, k, nx, ny);
-      lhz = hzp * plane + col;
-      if (hxk) { hx0 = ld_c(HX.a0, lhx, HX.n, st); hx1 = ld_c(HX.a1, lhx, HX.n, st); }
-      if (hyk) { hy0 = ld_c(HY.a0, lhy, HY.n, st); hy1 = ld_c(HY.a1, lhy, HY.n, st); }
-      if (hzp >= 0) { hz0 = ld_c(HZ.a0, lhz, HZ.n, st); hz1 = ld_c(HZ.a1, lhz, HZ.n, st); hzb = HZ.b[k]; }
+    }
+    if (fy) {
+      const int se = face_plane<1>(EY, k, nx, ny);
+      if (eyo >= 0 && k >= 1) face_w(EY, eyo + se, ld(EY.c + j + 1), ey0o, ey1o, st);
+      if (eyp >= 0 && k >= 1) face_w(EY, eyp + se, ld(EY.c + jp + 1), ey0p, ey1p, st);
+      if (hyo >= 0 && k >= HY.zlo) {
+        lhy = hyo + face_plane<1>(HY, k, nx, ny);
+        face_w(HY, lhy, R(1), hy0, hy1, st);
+      }
+    }
+    if (fz) {
+      const int ezo = face_pos(EZ, k), ezq = face_pos(EZ, k + 1);
+      if (ezo >= 0) face_w(EZ, ezo * int(pl) + int(col), ld(EZ.c + k), zw0, zw1, st);
+      if (ezq >= 0) face_w(EZ, ezq * int(pl) + int(col), ld(EZ.c + k + 1), ez0p, ez1p, st);
+      hzp = face_pos(HZ, k);
+      lhz = hzp * int(pl) + int(col);
+      if (hzp >= 0) face_w(HZ, lhz, R(1), hz0, hz1, st);
     }
     const bool obj = oxy && k == p.oz0;
     R oex = R(0), oey = R(0);
     if (obj) {
-      oex = ldg_c(p.En[0], c0, nf, st);
-      oey = ldg_c(p.En[1], c0, nf, st);
+      oex = at(p.En[0], base, col, nf, st);
+      oey = at(p.En[1], base, col, nf, st);
     }
 
     // ---- transposed curl_E and E faces
@@ -573,17 +579,18 @@ __device__ __forceinline__ void adj_b_cells(const AdjParams<T> &p, int bxi, int 
     b[0] += dt * (-kyj * gzk + kyp * gz_yp);
     // E faces: psi0 / psi1 feed (y, z) on x faces, (z, x) on y faces, (x, y) on
     // z faces; their differences of B run backward along the axis
-    if (fpl) {
+    if (fx) {
       b[2] += -ex0o + ex0p;
       b[1] += ex1o - ex1p;
+    }
+    if (fy) {
       b[0] += -ey0o + ey0p;
       b[2] += ey1o - ey1p;
+    }
+    if (fz) {
       b[1] += -zw0 + ez0p;
       b[0] += zw1 - ez1p;
     }
-    zw0 = ez0p;
-    zw1 = ez1p;
-    zw_on = ezq >= 0;
     // the objective's B term of the state before the step (Sz plane)
     if (obj) {
       b[0] -= p.obj_f_t * oey;
@@ -592,40 +599,28 @@ __device__ __forceinline__ void adj_b_cells(const AdjParams<T> &p, int bxi, int 
 
     // ---- stores: B adjoint, H-face totals for the step before (b * total + dt * B adjoint)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) st_c(p.Bb[c], c0, nf, st, T(b[c]));
-    if (fpl) {
-      if (hxk) {
-        st_c(HX.a0, lhx, HX.n, st, T(hxb * hx0 + dt * comp0<0>(b)));
-        st_c(HX.a1, lhx, HX.n, st, T(hxb * hx1 + dt * comp1<0>(b)));
-      }
-      if (hyk) {
-        st_c(HY.a0, lhy, HY.n, st, T(hyb * hy0 + dt * comp0<1>(b)));
-        st_c(HY.a1, lhy, HY.n, st, T(hyb * hy1 + dt * comp1<1>(b)));
-      }
-      if (hzp >= 0) {
-        st_c(HZ.a0, lhz, HZ.n, st, T(hzb * hz0 + dt * comp0<2>(b)));
-        st_c(HZ.a1, lhz, HZ.n, st, T(hzb * hz1 + dt * comp1<2>(b)));
-      }
-    }
+    for (int c = 0; c < 3; ++c) put(p.Bb[c], base, col, nf, st, b[c]);
+    if (fx && lhx >= 0) face_step(HX, lhx, ld(HX.b + i + 1), hx0, hx1, dt, comp0<0>(b), comp1<0>(b), st);
+    if (fy && lhy >= 0) face_step(HY, lhy, ld(HY.b + j + 1), hy0, hy1, dt, comp0<1>(b), comp1<1>(b), st);
+    if (fz && hzp >= 0) face_step(HZ, lhz, ld(HZ.b + k), hz0, hz1, dt, comp0<2>(b), comp1<2>(b), st);
     gx_k = gx_kp;
     gy_k = gy_kp;
   }
 }
 
 // The B half of the reverse step (blocks 0 .. nb-1 of a one-dimensional grid,
-// x fastest over gx x gy x z-chunks) and the design gradients of the step
-// (the blocks after them, over the design box in 32 x 4 tiles, one plane
-// each).
+// gx blocks a z-chunk) and the design gradients of the step (the blocks after
+// them, over the design box in tiles of 32 x kRowTile, one plane each).
 template <typename T, int NP, bool NL>
-__global__ void __launch_bounds__(MPB_ADJ_THREADS, (sizeof(T) == 4 ? MPB_ADJ_B_MIN_F : MPB_ADJ_B_MIN_D) / MPB_ADJ_THREADS)
-    adj_b_kernel(const AdjParams<T> p, const int gx, const int gy, const int nb) {
+__global__ void __launch_bounds__(kRowThreads, adj_b_threads<T>() / kRowThreads)
+    adj_b_kernel(const AdjParams<T> p, const AdjGrid g, const int gx, const int nb) {
   pdl_launch_dependents();
   const int b = blockIdx.x;
   if (b < nb) {
-    adj_b_cells<T>(p, b % gx, (b / gx) % gy, b / (gx * gy));
+    adj_b_cells<T>(p, g, b % gx, b / gx);
   } else {
     const int q = b - nb;
-    const int tx = (p.design.bx + 31) / 32, ty = (p.design.by + MPB_ADJ_BLOCK_Y - 1) / MPB_ADJ_BLOCK_Y;
+    const int tx = (p.design.bx + 31) / 32, ty = (p.design.by + kRowTile - 1) / kRowTile;
     adj_grad_cells<T, NP, NL>(p, q % tx, (q / tx) % ty, q / (tx * ty));
   }
 }
@@ -658,14 +653,14 @@ __global__ void __launch_bounds__(256) adj_init_kernel(const AdjParams<T> p) {
     st_c(p.Bb[c], c0, nf, st, T(b[c]));
   }
   // H-face totals: dt times the adjoint of B
-  const int hxo = face_pos(p.fh[0], i + 1), hyo = face_pos(p.fh[1], j + 1), hzo = face_pos(p.fh[2], k);
+  const int hxo = face_at<0>(p.fh[0], i, j, p.nx), hyo = face_at<1>(p.fh[1], i, j, p.nx), hzo = face_pos(p.fh[2], k);
   if (hxo >= 0 && k >= p.fh[0].zlo) {
-    const int li = face_col<0>(p.fh[0], hxo, i, j, p.nx) + face_plane<0>(p.fh[0], k, p.nx, p.ny);
+    const int li = hxo + face_plane<0>(p.fh[0], k, p.nx, p.ny);
     st_c(p.fh[0].a0, li, p.fh[0].n, st, T(p.dt * comp0<0>(b)));
     st_c(p.fh[0].a1, li, p.fh[0].n, st, T(p.dt * comp1<0>(b)));
   }
   if (hyo >= 0 && k >= p.fh[1].zlo) {
-    const int li = face_col<1>(p.fh[1], hyo, i, j, p.nx) + face_plane<1>(p.fh[1], k, p.nx, p.ny);
+    const int li = hyo + face_plane<1>(p.fh[1], k, p.nx, p.ny);
     st_c(p.fh[1].a0, li, p.fh[1].n, st, T(p.dt * comp0<1>(b)));
     st_c(p.fh[1].a1, li, p.fh[1].n, st, T(p.dt * comp1<1>(b)));
   }
@@ -731,16 +726,39 @@ __global__ void __launch_bounds__(256) sum_terms_kernel(const double *terms, lon
 // ---------------------------------------------------------------------------
 // Launchers
 
+// The grid of a reverse kernel over nk planes (zlo / zhi: set by the caller).
+// One plane per block on the smallest grids, up to 8 on large ones (reverse step
+// with 2 / 3 / 4 / 8 planes: 96^3 FP32 40 / 40 / 42 / 49 us, 120 x 104 x 136 FP64
+// Kerr 165 / 162 / 165 / 184, 256^3 FP32 Kerr 877 / 823 / 804 / 778; 64 x 56 x 70
+// with 1 / 2 / 3 21 / 23 / 26).  The next plane is prefetched into L2 where the
+// adjoint state does not stay there (256^3 855 -> 778 us, 192 x 192 x 256 FP64
+// 602 -> 546; 96^3 40 -> 41).
+template <typename T>
+static AdjGrid adj_grid(const AdjParams<T> &p, int nk, int *blocks) {
+  AdjGrid g;
+  static_cast<RowMap &>(g) = row_map(p.nx, p.ny, 1);
+  const long long bxy = (g.nvec + 31) / 32, all = bxy * nk;
+  *blocks = int(bxy);
+  g.kchunk = std::max(int(std::min(8LL, (all + 6499) / 6500)), (nk + 65534) / 65535);
+  g.ahead = (long long)sizeof(T) * (9 * p.n_field + 6 * p.np * p.n_psi) > (160LL << 20);
+  return g;
+}
+
 template <typename T>
 cudaError_t launch_adj_e(const AdjParams<T> &p, cudaStream_t st) {
-  const dim3 b(32, MPB_ADJ_BLOCK_Y, 1),
-      g((p.nx + 31) / 32, (p.ny + MPB_ADJ_BLOCK_Y - 1) / MPB_ADJ_BLOCK_Y, (p.nz + p.kchunk_e - 1) / p.kchunk_e);
+  int gx;
+  AdjGrid q = adj_grid(p, p.nz, &gx);
+  // planes k with k or k - 1 in an H layer, or k in an E layer
+  const AdjFace<T> &H = p.fh[2], &E = p.fe[2];
+  q.zlo = std::max(H.active ? H.hi0 + 1 : -1, E.active ? E.hi0 : -1);
+  q.zhi = std::min(H.active && H.lo1 <= H.hi1 ? H.lo1 : 1 << 30, E.active && E.lo1 <= E.hi1 ? E.lo1 : 1 << 30);
+  const dim3 b(kRowThreads, 1, 1), g(gx, (p.nz + q.kchunk - 1) / q.kchunk);
   const bool nl = p.nonlin != 0;
   switch (p.np) {
-    case 0: return nl ? launch_pdl(adj_e_kernel<T, 0, true>, g, b, st, p) : launch_pdl(adj_e_kernel<T, 0, false>, g, b, st, p);
-    case 1: return nl ? launch_pdl(adj_e_kernel<T, 1, true>, g, b, st, p) : launch_pdl(adj_e_kernel<T, 1, false>, g, b, st, p);
-    case 2: return nl ? launch_pdl(adj_e_kernel<T, 2, true>, g, b, st, p) : launch_pdl(adj_e_kernel<T, 2, false>, g, b, st, p);
-    default: return nl ? launch_pdl(adj_e_kernel<T, 3, true>, g, b, st, p) : launch_pdl(adj_e_kernel<T, 3, false>, g, b, st, p);
+    case 0: return nl ? launch_pdl(adj_e_kernel<T, 0, true>, g, b, st, p, q) : launch_pdl(adj_e_kernel<T, 0, false>, g, b, st, p, q);
+    case 1: return nl ? launch_pdl(adj_e_kernel<T, 1, true>, g, b, st, p, q) : launch_pdl(adj_e_kernel<T, 1, false>, g, b, st, p, q);
+    case 2: return nl ? launch_pdl(adj_e_kernel<T, 2, true>, g, b, st, p, q) : launch_pdl(adj_e_kernel<T, 2, false>, g, b, st, p, q);
+    default: return nl ? launch_pdl(adj_e_kernel<T, 3, true>, g, b, st, p, q) : launch_pdl(adj_e_kernel<T, 3, false>, g, b, st, p, q);
   }
 }
 
@@ -748,19 +766,22 @@ cudaError_t launch_adj_e(const AdjParams<T> &p, cudaStream_t st) {
 // extra blocks of the same launch.
 template <typename T>
 cudaError_t launch_adj_b(const AdjParams<T> &p, cudaStream_t st) {
-  const int gx = (p.nx + 31) / 32, gy = (p.ny + MPB_ADJ_BLOCK_Y - 1) / MPB_ADJ_BLOCK_Y,
-            gz = (p.nz + 1 + p.kchunk_b - 1) / p.kchunk_b;
-  const int nb = gx * gy * gz;
+  int gx;
+  AdjGrid q = adj_grid(p, p.nz + 1, &gx);
+  // planes k with k or k + 1 in an E layer, or k in an H layer
+  const AdjFace<T> &H = p.fh[2], &E = p.fe[2];
+  q.zlo = std::max(H.active ? H.hi0 : -1, E.active ? E.hi0 : -1);
+  q.zhi = std::min(H.active && H.lo1 <= H.hi1 ? H.lo1 : 1 << 30, E.active && E.lo1 <= E.hi1 ? E.lo1 - 1 : 1 << 30);
+  const int nb = gx * ((p.nz + 1 + q.kchunk - 1) / q.kchunk);
   const DesignParams &d = p.design;
-  const int ng = d.x0 <= d.x1 ? ((d.bx + 31) / 32) * ((d.by + MPB_ADJ_BLOCK_Y - 1) / MPB_ADJ_BLOCK_Y) * (d.z1 - d.z0 + 1)
-                              : 0;
-  const dim3 b(32, MPB_ADJ_BLOCK_Y, 1), g(nb + ng, 1, 1);
+  const int ng = d.x0 <= d.x1 ? ((d.bx + 31) / 32) * ((d.by + kRowTile - 1) / kRowTile) * (d.z1 - d.z0 + 1) : 0;
+  const dim3 b(kRowThreads, 1, 1), g(nb + ng, 1, 1);
   const bool nl = p.nonlin != 0;
   switch (p.np) {
-    case 0: return nl ? launch_pdl(adj_b_kernel<T, 0, true>, g, b, st, p, gx, gy, nb) : launch_pdl(adj_b_kernel<T, 0, false>, g, b, st, p, gx, gy, nb);
-    case 1: return nl ? launch_pdl(adj_b_kernel<T, 1, true>, g, b, st, p, gx, gy, nb) : launch_pdl(adj_b_kernel<T, 1, false>, g, b, st, p, gx, gy, nb);
-    case 2: return nl ? launch_pdl(adj_b_kernel<T, 2, true>, g, b, st, p, gx, gy, nb) : launch_pdl(adj_b_kernel<T, 2, false>, g, b, st, p, gx, gy, nb);
-    default: return nl ? launch_pdl(adj_b_kernel<T, 3, true>, g, b, st, p, gx, gy, nb) : launch_pdl(adj_b_kernel<T, 3, false>, g, b, st, p, gx, gy, nb);
+    case 0: return nl ? launch_pdl(adj_b_kernel<T, 0, true>, g, b, st, p, q, gx, nb) : launch_pdl(adj_b_kernel<T, 0, false>, g, b, st, p, q, gx, nb);
+    case 1: return nl ? launch_pdl(adj_b_kernel<T, 1, true>, g, b, st, p, q, gx, nb) : launch_pdl(adj_b_kernel<T, 1, false>, g, b, st, p, q, gx, nb);
+    case 2: return nl ? launch_pdl(adj_b_kernel<T, 2, true>, g, b, st, p, q, gx, nb) : launch_pdl(adj_b_kernel<T, 2, false>, g, b, st, p, q, gx, nb);
+    default: return nl ? launch_pdl(adj_b_kernel<T, 3, true>, g, b, st, p, q, gx, nb) : launch_pdl(adj_b_kernel<T, 3, false>, g, b, st, p, q, gx, nb);
   }
 }
 

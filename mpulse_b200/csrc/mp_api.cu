@@ -51,12 +51,6 @@ cudaError_t launch_b_half_tma(const BParams<T> &, const BTmaMaps &, cudaStream_t
 template <typename T>
 cudaError_t launch_step_fused(const EParams<T> &, const BParams<T> &, int, int, int, cudaStream_t);
 void tma_boxes(int esz, int e_box[7][2], int b_box[6][2]);
-#ifndef MPB_ADJ_E_BPSM
-#define MPB_ADJ_E_BPSM 8
-#endif
-#ifndef MPB_ADJ_B_BPSM
-#define MPB_ADJ_B_BPSM 8
-#endif
 template <typename T> cudaError_t launch_adj_e(const AdjParams<T> &, cudaStream_t);
 template <typename T> cudaError_t launch_adj_b(const AdjParams<T> &, cudaStream_t);
 template <typename T> cudaError_t launch_adj_init(const AdjParams<T> &, cudaStream_t);
@@ -1598,6 +1592,7 @@ int adj_faces(mp_ctx *c, DevBufs &buf, bool isH, const CpmlFace<T> *fw, AdjFace<
   for (int dim = 0; dim < 3; ++dim) {
     AdjFace<T> &F = out[dim];
     F = AdjFace<T>();
+    F.lo0 = F.lo1 = 1;
     int fl[2], nf = 0;
     for (int f = 0; f < 6; ++f) {
       const LayerHost &L = isH ? c->cpH[f] : c->cpE[f];
@@ -2051,19 +2046,6 @@ int adjoint_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const mp_adjoint_con
   p.n_field = (long long)c->fcount;
   p.n_psi = (long long)c->psi_cells;
   p.n_design = (long long)c->dcells;
-  {
-    // planes per block: about MPB_ADJ_E_BPSM / MPB_ADJ_B_BPSM blocks of 32 x 4
-    // columns per SM (measured on the 96^3 adjoint workload, FP32: for adj_e
-    // 6 planes per block beat 3 and 2)
-    const long long blocks_xy = (long long)((g.nx + 31) / 32) * ((g.ny + 3) / 4);
-    const long long ce = std::max(1LL, (148LL * MPB_ADJ_E_BPSM + blocks_xy - 1) / blocks_xy);
-    const long long cb = std::max(1LL, (148LL * MPB_ADJ_B_BPSM + blocks_xy - 1) / blocks_xy);
-    p.kchunk_e = int(std::max(1LL, (g.nz + ce - 1) / ce));
-    p.kchunk_b = int(std::max(1LL, (g.nz + 1 + cb - 1) / cb));
-#ifdef MPB_ADJ_KCHUNK
-    p.kchunk_e = p.kchunk_b = MPB_ADJ_KCHUNK;
-#endif
-  }
   p.plane = c->plane;
   p.dt = g.dt;
   for (int q = 0; q < 3; ++q) {

@@ -203,7 +203,6 @@ struct AdjParams {
   T pDt[3][2], pxit[3][2], pCt[3][2];
   T inv_eps_bg_t, eps_bg_t, numer0_t, inv_denom0_t, chi_nl_t, obj_f_t;
   int np, mz0, mz1, nonlin;
-  int kchunk_e, kchunk_b;  // planes per block of adj_e (1..nz) / adj_b (0..nz)
   AdjFace<T> fe[3], fh[3];  // per axis x, y, z
   DesignParams design;
   double *grad[3];        // dJ/d eps, dJ/d Delta-eps factor, dJ/d chi factor (box-sized, FP64)

@@ -13,6 +13,8 @@ namespace mpb {
 constexpr int kRowTile = 4;
 constexpr int kRowThreads = 32 * kRowTile;
 
+__device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
+
 // V consecutive elements of a row.
 template <typename T, int V>
 struct alignas(sizeof(T) * V <= 16 ? sizeof(T) * V : 16) RowV {

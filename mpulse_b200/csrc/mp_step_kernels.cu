@@ -62,8 +62,6 @@ __host__ __device__ constexpr int b_threads(bool early) {
   return sizeof(T) == 8 ? 768 : early ? 768 : 1280;
 }
 
-__device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
-
 // What a half step's grid needs beside the row mapping.
 struct HalfGrid : RowMap {
   int kchunk;           // planes per block
