@@ -173,6 +173,7 @@ struct mp_ctx {
   void *plasma[4] = {nullptr, nullptr, nullptr, nullptr};  // PlasmaDensity, PlasmaJx, PlasmaJy, PlasmaJz
   int *d_status = nullptr;
   int *h_status = nullptr;
+  volatile int *h_flag = nullptr;  // raised by the first error a kernel counts
   unsigned long long *d_kerr = nullptr;  // Kerr solves and Newton iterations since the last mp_kerr_counts
   unsigned long long *h_kerr = nullptr;
   double *staging = nullptr;
@@ -200,6 +201,7 @@ struct mp_ctx {
     cudaGraphExec_t exec;
   };
   std::vector<StepGraph> graphs;
+  std::vector<std::pair<const void *, int>> graph_seen;  // (planes, K) that came once
   bool use_graphs = false;
   ETmaMaps etma;
   BTmaMaps btma;
@@ -780,7 +782,7 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
     }
   }
   c->mem.want(&c->lines, host_lines.size() * c->esz);
-  c->mem.want(&c->d_status, ST_COUNT * sizeof(int));
+  c->mem.want(&c->d_status, ST_COUNT * sizeof(int) + sizeof(int *));
   c->mem.want(&c->d_kerr, kKerrBytes);
   c->mem.want(&c->d_diag, size_t(g.nz + 3) * sizeof(double));
   c->mem.want(&c->d_terms, kTerms * sizeof(double));
@@ -806,11 +808,17 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
             "cudaMemcpy");
     MPB_TRY(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
   }
-  // the pinned results: the Kerr counters, two doubles, the status word
-  MPB_TRY(cudaMallocHost(&c->pinned, kKerrBytes + 2 * sizeof(double) + ST_COUNT * sizeof(int)), "pinned allocation");
+  // the pinned results: the Kerr counters, two doubles, the status word, its flag
+  MPB_TRY(cudaMallocHost(&c->pinned, kKerrBytes + 2 * sizeof(double) + (ST_COUNT + 1) * sizeof(int)), "pinned allocation");
   c->h_kerr = static_cast<unsigned long long *>(c->pinned);
   c->h_diag = reinterpret_cast<double *>(static_cast<char *>(c->pinned) + kKerrBytes);
   c->h_status = reinterpret_cast<int *>(c->h_diag + 2);
+  c->h_flag = c->h_status + ST_COUNT;
+  *c->h_flag = 0;
+  int *flag = nullptr;
+  MPB_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&flag), c->h_status + ST_COUNT, 0), "cudaHostGetDevicePointer");
+  MPB_TRY(cudaMemcpyAsync(c->d_status + ST_COUNT, &flag, sizeof flag, cudaMemcpyHostToDevice, c->stream), "cudaMemcpy");
+  MPB_TRY(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
 
   if (c->fp32) build_params<float>(c, c->epf, c->bpf, ikE_off, ikH_off, bzy_off, coef, numer, denom);
   else build_params<double>(c, c->epd, c->bpd, ikE_off, ikH_off, bzy_off, coef, numer, denom);
@@ -850,8 +858,9 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
   // (E 1.12 ms, B 0.61 ms), whose 12 small tile copies per plane and block
   // serialise in the copy engine.
   c->fused = g.staging == MP_STAGING_FUSED;
-  // CUDA graphs for grids of up to 4 M cells, whose half steps take a few
-  // microseconds, so that the gaps between launches matter
+  // CUDA graphs for grids of up to 4 M cells, where the gaps between launches
+  // matter (50 steps of 64^3 FP32 346 instead of 399 us, one step of 32^3 FP64 12
+  // instead of 19, 20 steps of 150 x 131 x 210 FP32 960 instead of 1000)
   c->use_graphs = (long long)g.nx * g.ny * g.nz <= (4LL << 20);
   if (g.staging == MP_STAGING_TMA) {
     if (!setup_tma(c)) return fail(set_err(c, MP_ERR_UNSUPPORTED, "TMA tensor maps could not be encoded"));
@@ -1027,11 +1036,11 @@ cudaError_t launch_steps(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const T *pla
   return cudaSuccess;
 }
 
-// The graph of K steps from `planes`, captured on first use (the kernels'
+// The graph of K steps from `planes`, captured on second use (the kernels'
 // parameters are fixed for the context but for the injection planes; the
-// plane buffers are read when the graph runs).  *exec = nullptr when the
-// stream is being captured by the caller (the steps are then launched one by
-// one, into the caller's graph).
+// plane buffers are read when the graph runs).  *exec = nullptr on first use and
+// when the stream is being captured by the caller (the steps are then launched
+// one by one, into the caller's graph).
 template <typename T>
 int step_graph(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const T *planes, int K, cudaGraphExec_t *exec) {
   *exec = nullptr;
@@ -1044,6 +1053,15 @@ int step_graph(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const T *planes, int K
       *exec = g.exec;
       return MP_OK;
     }
+  // captured the second time: a batch that comes once would pay for the capture
+  // (a first pass of 20 steps 1015 us, with capture 1190)
+  bool seen = false;
+  for (const auto &q : c->graph_seen) seen = seen || (q.first == planes && q.second == K);
+  if (!seen) {
+    if (c->graph_seen.size() >= 16) c->graph_seen.erase(c->graph_seen.begin());
+    c->graph_seen.emplace_back(planes, K);
+    return MP_OK;
+  }
   if (c->graphs.size() >= 16) {  // keep the most recent ones
     cudaGraphExecDestroy(c->graphs.front().exec);
     c->graphs.erase(c->graphs.begin());
@@ -1114,7 +1132,11 @@ int step_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, int n_steps, StepTimer 
         acc[2] += ms;  // sources, all steps of the block
       }
     }
-    if (c->use_graphs && !tm && !hooks) {
+    // With an injector a graph holds the addresses of its steps' planes, so only
+    // whole batches, which start at one of two, are replayed; others come at too
+    // many offsets (20 steps of 128^3 with every batch captured 1373 us, launched one
+    // by one 1144).
+    if (c->use_graphs && !tm && !hooks && (!c->nsrc || K == c->src_batch)) {
       // the batch as one CUDA graph (at most 64 steps per graph)
       const int Kg = std::min(K, 64);
       cudaGraphExec_t g;
@@ -1408,7 +1430,11 @@ int mp_step_async(mp_ctx *c, int n_steps) {
 int mp_check_status(mp_ctx *c) {
   if (!c) return MP_ERR_INVALID;
   cudaSetDevice(c->cfg.device);
-  cudaError_t e = cudaMemcpyAsync(c->h_status, c->d_status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return cuda_err(c, e, "status read");
+  if (!*c->h_flag) return MP_OK;
+  *c->h_flag = 0;
+  e = cudaMemcpyAsync(c->h_status, c->d_status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "status read");
   const int newton = c->h_status[ST_NEWTON], nonfin = c->h_status[ST_NONFINITE];

@@ -112,7 +112,7 @@ __device__ __forceinline__ double kerr_newton(double E, double A, double C, doub
     E = (2.0 * A * E2 * E + C) * (FP32 ? rcp_pos1(d) : rcp_pos(d));
     ++it;
   } while (fabs(E - Eold) > tol && it < maxit);
-  if (fabs(E - Eold) > tol) atomicAdd(status + ST_NEWTON, 1);
+  if (fabs(E - Eold) > tol) report(status, ST_NEWTON);
   *iters += unsigned(it);
   return E;
 }
@@ -128,7 +128,7 @@ __device__ __forceinline__ double nl_newton(double E, double eps, double chi, do
     E = (2.0 * chi * E2 * E + D) * rcp_pos(3.0 * chi * E2 + eps);
     ++it;
   } while (fabs(E - Eold) > tol && it < maxit);
-  if (fabs(E - Eold) > tol) atomicAdd(status + ST_NEWTON, 1);
+  if (fabs(E - Eold) > tol) report(status, ST_NEWTON);
   *iters += unsigned(it);
   return E;
 }
@@ -460,7 +460,7 @@ __device__ __forceinline__ void e_update(const EParams<T> &p, const CellCoef<T, 
       }
     }
   }
-  if (!finite3(exn, eyn, ezn)) atomicAdd(p.status + ST_NONFINITE, 1);
+  if (!finite3(exn, eyn, ezn)) report(p.status, ST_NONFINITE);
 }
 
 // SPECIAL = false: the caller guarantees that no CPML face contains the cell

@@ -9,6 +9,12 @@
 
 namespace mpb {
 
+// Counts an error in the status word and, when it is the slot's first, raises the
+// host's flag, whose address follows the counts (StatusSlot).
+__device__ __forceinline__ void report(int *status, int slot) {
+  if (atomicAdd(status + slot, 1) == 0) **reinterpret_cast<volatile int *const *>(status + ST_COUNT) = 1;
+}
+
 // A checked build (MPB_CHECKED=1, the library libmpulse_b200_checked.so)
 // tests every element index against the size of its array; an index outside
 // is counted in the status word (ST_BOUNDS, reported by mp_step / mp_adjoint
@@ -20,7 +26,7 @@ namespace mpb {
 __device__ __forceinline__ bool in_bounds(long long i, long long n, int *status) {
 #if MPB_CHECKED
   if ((unsigned long long)i < (unsigned long long)n) return true;
-  atomicAdd(status + ST_BOUNDS, 1);
+  report(status, ST_BOUNDS);
   return false;
 #else
   (void)i;

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (k0 > k1) return;  // whole block
   const int nplanes = k1 - k0 + 1;
   if (smem_u32(smem) & 127) {  // tile copies need 128-byte aligned destinations
-    if (tx == 0 && ty == 0) atomicAdd(p.status + ST_TIMEOUT, 1);
+    if (tx == 0 && ty == 0) report(p.status, ST_TIMEOUT);
     return;
   }
   if (tx == 0 && ty == 0) {
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int m = 0; m < nplanes; ++m) {
       const int s = m % S;
       if (m >= S && !mbar_wait(&empty[s], ((m / S) + 1) & 1)) {
-        atomicAdd(p.status + ST_TIMEOUT, 1);
+        report(p.status, ST_TIMEOUT);
         return;
       }
       const int k = k0 + m;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int k = k0 + m;
     const int s = m % S;
     if (!mbar_wait(&full[s], (m / S) & 1)) {
-      if (tx == 0) atomicAdd(p.status + ST_TIMEOUT, 1);
+      if (tx == 0) report(p.status, ST_TIMEOUT);
       return;
     }
     const unsigned char *st = smem + s * L::STAGE;
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   // planes k0 .. k1 + 1 are loaded (the last only for its Ex, Ey)
   const int nload = k1 - k0 + 2;
   if (smem_u32(smem) & 127) {
-    if (tx == 0 && ty == 0) atomicAdd(p.status + ST_TIMEOUT, 1);
+    if (tx == 0 && ty == 0) report(p.status, ST_TIMEOUT);
     return;
   }
   if (tx == 0 && ty == 0) {
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int m = 0; m < nload; ++m) {
       const int s = m % S;
       if (m >= S && !mbar_wait(&empty[s], ((m / S) + 1) & 1)) {
-        atomicAdd(p.status + ST_TIMEOUT, 1);
+        report(p.status, ST_TIMEOUT);
         return;
       }
       int k = k0 + m;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // plane k0's centre values of Ex, Ey, carried as "this plane" into the loop
   if (!mbar_wait(&full[0], 0)) {
-    if (tx == 0) atomicAdd(p.status + ST_TIMEOUT, 1);
+    if (tx == 0) report(p.status, ST_TIMEOUT);
     return;
   }
   T ex_k = reinterpret_cast<const T *>(smem + L::oEX)[ty * kTX + tx];
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int s = m % S, sn = (m + 1) % S;
     // stage s (plane k) is complete since the previous iteration; wait for k+1
     if (!mbar_wait(&full[sn], ((m + 1) / S) & 1)) {
-      if (tx == 0) atomicAdd(p.status + ST_TIMEOUT, 1);
+      if (tx == 0) report(p.status, ST_TIMEOUT);
       return;
     }
     const unsigned char *st = smem + s * L::STAGE;
