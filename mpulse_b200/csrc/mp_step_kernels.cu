@@ -611,21 +611,28 @@ static cudaError_t launch_e_v(const EParams<T> &p, int np, cudaStream_t st) {
   constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
   dim3 d;
   const HalfGrid g = row_grid(p, V, max_planes<T>(), &d);
-  return PLRC && g.apart ? launch_e_np<T, V, MODE, DESIGN, PLASMA, PLRC>(p, np, g, d, st)
+  constexpr bool EARLY = PLRC && !(MODE == MODE_PLRC_NONLIN && V == 2);
+  return EARLY && g.apart ? launch_e_np<T, V, MODE, DESIGN, PLASMA, EARLY>(p, np, g, d, st)
                          : launch_e_np<T, V, MODE, DESIGN, PLASMA, false>(p, np, g, d, st);
 }
 
 // Two cells per thread in FP32 where the update is short (150 x 131 x 210
 // fdtd-plain 30 instead of 38 us, 160 x 144 x 250 PLRC with one pole 79 instead
 // of 81, 128^3 with two poles 46 instead of 49), but not with two poles and x / y
-// layers (160 x 144 x 250 124 us with one cell, 141 with two); one with Kerr or the plasma
-// plug-ins (128 x 128 x 256 Kerr 108 instead of 113 us, 128 x 128 x 192 plasma
-// 109 instead of 116), with a design region (96^3 21.6 instead of 23.0) and in
-// FP64, whose two-cell form spills (192 x 192 x 384 551 instead of 691 us).
+// layers (160 x 144 x 250 124 us with one cell, 141 with two); one with the plasma
+// plug-ins (128 x 128 x 192 109 instead of 116), with a design region (96^3 21.6
+// instead of 23.0) and in FP64, whose two-cell form spills (192 x 192 x 384 551
+// instead of 691 us).  With Kerr one cell is faster by itself (128 x 128 x 256 102
+// instead of 114 us, 256 x 256 x 512 666 instead of 677), but two cells issue a
+// fifth fewer instructions: states above 1 GB, which keep the GPU at its power
+// limit, take two (256 x 256 x 512, 400 steps on end: 1032 us a step with one,
+// 1007 with two), and without the early face loads, for which it lacks registers
+// (827 us).
 template <typename T, int MODE, bool DESIGN, bool PLASMA>
 static cudaError_t launch_e(const EParams<T> &p, int np, cudaStream_t st) {
-  constexpr int V = sizeof(T) == 4 && MODE != MODE_PLRC_NONLIN && !DESIGN && !PLASMA ? 2 : 1;
-  const bool two = p.nx % V == 0 && p.nx > V && !(np >= 2 && xy_faces(p));
+  constexpr int V = sizeof(T) == 4 && !DESIGN && !PLASMA ? 2 : 1;
+  const bool two = p.nx % V == 0 && p.nx > V &&
+                   (MODE == MODE_PLRC_NONLIN ? p.state_bytes > (1LL << 30) : !(np >= 2 && xy_faces(p)));
   return two ? launch_e_v<T, V, MODE, DESIGN, PLASMA>(p, np, st)
                                    : launch_e_v<T, 1, MODE, DESIGN, PLASMA>(p, np, st);
 }

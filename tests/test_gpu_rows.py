@@ -5,7 +5,7 @@ shorter last one, CPML layers that meet or overlap, with an injection plane; aga
 the CPU oracle, to the suite's bars (FP64 1e-12, FP32 1e-5 relative L2)."""
 import pytest
 
-from mpulse_b200 import abi, runtime
+from mpulse_b200 import abi, configs, runtime
 from oracle import pyoracle
 from tests.cases import make_case, random_fields, rel_l2
 
@@ -37,3 +37,23 @@ def test_rows_match_oracle(case, shape, precision, tol):
         g.step(12)
         for n in abi.FIELD_NAMES:
             assert rel_l2(g.download(n), o.download(n)) <= tol, n
+
+
+def test_large_kerr_state_fp32_matches_fp64():
+    """A state above 1 GB in FP32 (its E half runs two cells per thread, and both
+    halves prefetch the next plane) against the FP64 form, on the workload's grid cut
+    to 240 planes: eight steps from a pulse in the Kerr medium, the FP32 bar of
+    1e-5."""
+    fields = {}
+    for precision in (abi.MP_FP64, abi.MP_FP32):
+        cfg = configs.c3_plrc_kerr(precision, nz=240, focus_z=120)
+        init = abi.default_init(abi.MP_INIT_PULSE)
+        init.k[:] = (0.0, 0.0, 2 * 3.141592653589793 / 0.8)
+        init.B[:] = (0.3, 1.0, 0.0)
+        init.r0, init.z0, init.zc, init.C = 2.0, 2.5, 150 * cfg.dz, 0.0
+        with runtime.Simulation(cfg) as g:
+            g.initialize(init)
+            g.step(8)
+            fields[precision] = {n: g.download(n) for n in abi.FIELD_NAMES}
+    for n in abi.FIELD_NAMES:
+        assert rel_l2(fields[abi.MP_FP32][n], fields[abi.MP_FP64][n]) <= 1e-5, n
