@@ -38,6 +38,7 @@ template <typename T> cudaError_t launch_e_half(const EParams<T> &, int, int, cu
 template <typename T> cudaError_t launch_b_half(const BParams<T> &, cudaStream_t);
 template <typename T>
 cudaError_t launch_source_batch(const SourceEvalParams &, const SourceEvalParams &, long long, int, T *, cudaStream_t);
+int source_batch_launches(const SourceEvalParams &);
 cudaError_t launch_convert_in(const double *src, void *dst, int fp32, long long n, int stride, int offset,
                               cudaStream_t st);
 cudaError_t launch_convert_out(const void *src, double *dst, int fp32, long long n, int stride, int offset,
@@ -978,7 +979,7 @@ int sources_ahead(mp_ctx *c, int want, const T **planes, int *steps) {
       return cuda_err(c, e, "cudaStreamWaitEvent");
     e = launch_source_batch<T>(c->sq[0][0], c->sq[0][1], c->time, c->src_batch, bufs[0], c->stream);
     if (e != cudaSuccess) return cuda_err(c, e, "source kernel");
-    c->launches++;
+    c->launches += source_batch_launches(c->sq[0][0]);
     c->pre_t0[0] = c->time;
     c->pre_k[0] = c->src_batch;
     c->pre_pending[0] = false;
@@ -1001,7 +1002,7 @@ int sources_ahead(mp_ctx *c, int want, const T **planes, int *steps) {
     e = launch_source_batch<T>(c->sq[0][0], c->sq[0][1], nt0, c->src_batch, bufs[w], c->src_stream);
     if (e != cudaSuccess) return cuda_err(c, e, "source kernel");
     if ((e = cudaEventRecord(c->src_done[w], c->src_stream)) != cudaSuccess) return cuda_err(c, e, "event");
-    c->launches++;
+    c->launches += source_batch_launches(c->sq[0][0]);
     c->pre_t0[w] = nt0;
     c->pre_k[w] = c->src_batch;
     c->pre_pending[w] = true;
@@ -1125,7 +1126,7 @@ int step_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, int n_steps, StepTimer 
       }
       e = launch_source_batch<T>(c->sq[0][0], c->sq[0][1], c->time, K, static_cast<T *>(c->src_buf), c->stream);
       if (e != cudaSuccess) return cuda_err(c, e, "source kernel");
-      c->launches++;
+      c->launches += source_batch_launches(c->sq[0][0]);
       if (tm) {
         cudaEventRecord(tm->ev[5], c->stream);
         e = cudaEventSynchronize(tm->ev[5]);
