@@ -411,7 +411,9 @@ void build_params(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const std::vector<s
     ep.pl_m = T(g.dt * g.plasma_mpa);
     ep.pl_w = T(g.plasma_mpa * g.plasma_wion);
     ep.pl_gdtn = T(1 - 0.5 * g.plasma_gamma * g.dt);
-    ep.pl_gdtd = T(1 + 0.5 * g.plasma_gamma * g.dt);
+    const T gd = T(1 + 0.5 * g.plasma_gamma * g.dt);
+    ep.pl_igd = T(1.0L / (long double)gd);
+    ep.pl_igd_lo = T(1.0L / (long double)gd - (long double)ep.pl_igd);
     ep.pl_emdt = T(g.plasma_em * g.dt);
     ep.pl_rho_bg = T(g.plasma_rho_bg);
   }

@@ -250,9 +250,12 @@ __device__ __forceinline__ void plasma_cell(const EParams<T> &p, T ex, T ey, T e
   }
   if (p.pl_current) {
     const T r = pc.rho + p.pl_rho_bg;
-    pc.j[0] = fma_pm(j0, p.pl_gdtn, p.pl_emdt * ex, r) / p.pl_gdtd;
-    pc.j[1] = fma_pm(j1, p.pl_gdtn, p.pl_emdt * ey, r) / p.pl_gdtd;
-    pc.j[2] = fma_pm(j2, p.pl_gdtn, p.pl_emdt * ez, r) / p.pl_gdtd;
+    // the division by 1 + gamma dt / 2 as a product with its reciprocal (hi + lo)
+    const T c0 = fma_pm(j0, p.pl_gdtn, p.pl_emdt * ex, r), c1 = fma_pm(j1, p.pl_gdtn, p.pl_emdt * ey, r),
+            c2 = fma_pm(j2, p.pl_gdtn, p.pl_emdt * ez, r);
+    pc.j[0] = fma(c0, p.pl_igd, c0 * p.pl_igd_lo);
+    pc.j[1] = fma(c1, p.pl_igd, c1 * p.pl_igd_lo);
+    pc.j[2] = fma(c2, p.pl_igd, c2 * p.pl_igd_lo);
   } else {
     pc.j[0] = pc.j[1] = pc.j[2] = T(0);
   }
@@ -340,7 +343,8 @@ __device__ __forceinline__ void plasma_coef(const EParams<T> &p, T sig, CellCoef
   lc.numer = lc.numer - sig;
   lc.inv_denom = T(1) / (p.denom_t + sig);
   lc.inv_denom_lo = T(0);
-  lc.chi_over_denom = p.chi_raw / (p.denom_d + (double)sig);
+  const double d = p.denom_d + (double)sig;
+  lc.chi_over_denom = p.chi_raw * (sizeof(T) == 4 ? rcp_pos1(d) : rcp_pos(d));
 }
 
 // The E update of one cell from its old E, the curl of B and the current sum:

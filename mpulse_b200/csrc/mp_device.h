@@ -144,7 +144,8 @@ struct EParams {
   int pl_density, pl_current;
   int pl_km;                        // K - 1
   T pl_n, pl_m, pl_w;               // dt nu / 2, dt mpa, mpa Wion
-  T pl_gdtn, pl_gdtd, pl_emdt, pl_rho_bg;  // 1 - gamma dt / 2, 1 + gamma dt / 2, em dt, rho_bg
+  T pl_gdtn, pl_emdt, pl_rho_bg;    // 1 - gamma dt / 2, em dt, rho_bg
+  T pl_igd, pl_igd_lo;              // 1 / (1 + gamma dt / 2), rounded, and the rest
   T denom_t;                        // the medium's denominator without the conductivity
   double denom_d, chi_raw;          // the same in FP64, and chi
 };
