@@ -13,9 +13,14 @@
 
 namespace mpb {
 
-// Let the next kernel of the stream start its blocks once all of this kernel's
-// have started, and wait until the previous kernel's writes are visible.  Both
-// are no-ops for a kernel launched without the attribute.
+// pdl_launch_dependents lets the next kernel of the stream start its blocks once
+// all of this kernel's have called it or ended; pdl_wait waits until the previous
+// kernel's writes are visible.  Both are no-ops for a kernel launched without the
+// attribute.  The step kernels call the first when a block has done its planes: called
+// at their start, the next kernel's blocks took the register file's room beside them
+// and waited there (64^3 FP32 6.9 us a step, at the end 5.8; 48^3 Kerr 7.7 and 6.3;
+// 32^3 FP64 4.2 and 3.6).  The reverse kernels, whose set-up is longer, call it at
+// their start (96^3 FP32 39.8 us a reverse step, at the end 46.5).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

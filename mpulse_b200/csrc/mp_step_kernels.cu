@@ -277,7 +277,6 @@ __global__ void __launch_bounds__(kRowThreads, e_threads<T>(V, PLASMA) / kRowThr
     e_half_kernel(const EParams<T> p, const HalfGrid g) {
   typedef typename Vec2<T>::type T2;
   constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
-  pdl_launch_dependents();
   const int nx = p.nx, ny = p.ny;
   int i0, j;  // 0-based: MPulse i + 1, j + 1
   if (!row_cells<V>(g, blockIdx.x, ny, i0, j)) return;
@@ -447,6 +446,7 @@ __global__ void __launch_bounds__(kRowThreads, e_threads<T>(V, PLASMA) / kRowThr
     bx_km = bx;
     by_km = by;
   }
+  pdl_launch_dependents();
   flush_kerr_count<MODE>(p.kerr_count, kc);
 }
 
@@ -456,7 +456,6 @@ __global__ void __launch_bounds__(kRowThreads, b_threads<T>(EARLY) / kRowThreads
   // the chunks from the top down: the E half wrote the top planes last, and
   // what of them is still in L2 is read from there (2-6% of both halves on grids
   // of up to twice the L2)
-  pdl_launch_dependents();
   const int nx = p.nx, ny = p.ny;
   int i0, j;
   if (!row_cells<V>(g, blockIdx.x, ny, i0, j)) return;
@@ -547,6 +546,7 @@ __global__ void __launch_bounds__(kRowThreads, b_threads<T>(EARLY) / kRowThreads
     ex = ex_kp;
     ey = ey_kp;
   }
+  pdl_launch_dependents();
 }
 
 // ---------------------------------------------------------------------------
@@ -559,7 +559,7 @@ static bool xy_faces(const P &p) {
 
 // The grid of a half step: V cells per thread, z-chunks of the planes.
 // Planes per block: one where two would leave SMs without four blocks (32^3
-// FP64: E 9.1 instead of 10.2 us); else at least two, and more while 50 blocks
+// FP64: E 9.1 instead of 10.2 us; 72^3 12.2 instead of 13.1 us a step); else at least two, and more while 50 blocks
 // per SM remain, up to max_planes.  Longer chunks save the two carried loads of
 // each chunk's first plane but leave fewer warps and a longer tail (256 x 256 x
 // 512 FP32 E half with 2 / 4 / 8 / 16 / 24 planes 725 / 682 / 677 / 700 / 715 us,
@@ -580,15 +580,15 @@ static HalfGrid row_grid(const P &p, int V, int max_planes, dim3 *d) {
   r.src = p.n_src > 0 ? p.src[0].plane : -1;
   const int nk = p.k_last - p.k_first + 1;
   const long long bxy = (r.nvec + 31) / 32, all = bxy * nk;
-  r.kchunk = all < 2 * 148 * 4 ? 1 : int(std::min<long long>(std::max(2LL, all / (148 * 50)), max_planes));
+  r.kchunk = all < 1600 ? 1 : int(std::min<long long>(std::max(2LL, all / (148 * 50)), max_planes));
   r.kchunk = std::max(r.kchunk, (nk + 65534) / 65535);  // blocks in y
   r.ahead = p.state_bytes > (160LL << 20);
   *d = dim3(unsigned(bxy), unsigned((nk + r.kchunk - 1) / r.kchunk), 1);
   return r;
 }
 
-// (Both kernels go out with programmatic dependent launch: 32^3 FP64 6.0 -> 5.2
-// us per step, 64^3 FP32 9.1 -> 8.7.)
+// (Both kernels go out with programmatic dependent launch: 32^3 FP64 6.0 -> 3.6
+// us per step, 64^3 FP32 9.1 -> 5.8.)
 template <typename T>
 constexpr int max_planes() {
   return sizeof(T) == 4 ? 8 : 4;
