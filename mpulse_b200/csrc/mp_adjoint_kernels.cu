@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kRowThreads, adj_e_threads<T>() / kRowThreads)
         prefetch_l2(p.Eb[c] + bn + col);
         if (NL) prefetch_l2(p.En[c] + bn + col);
         if (NL) prefetch_l2(p.En1[c] + bn + col);
-        if (med) {
+        if (med && k < p.mz1) {
 #pragma unroll
           for (int n = 0; n < NP; ++n)
             prefetch_l2(reinterpret_cast<const T2 *>(p.psib[n][c]) + pbase + pl + col);

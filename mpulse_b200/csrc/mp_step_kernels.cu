@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kRowThreads, e_threads<T>(V, PLASMA) / kRowThr
       prefetch_l2(Ex + ba + col);
       prefetch_l2(Ey + ba + col);
       prefetch_l2(Ez + ba + col);
-      if (NP > 0 && med) {
+      if (NP > 0 && med && k < p.mz1) {
 #pragma unroll
         for (int n = 0; n < NP; ++n)
 #pragma unroll
