@@ -103,16 +103,20 @@ __device__ __forceinline__ double rcp_pos1(double d) {
 // radians a step takes three.  256 x 256 x 512 Kerr FP32, steps on end at the power
 // limit: 1008 -> 967 us a step; E half of 128 x 128 x 192 with the plasma plug-ins 111
 // -> 104 us.
+// A < 0 always starts from |E^n|, as MPulse does (fdtd_plrc.cpp:406, fdtd_nl.cpp:86):
+// then E + A E^3 = C has three real roots, and the start decides which one is found.
+// (A static field with |A| E^2 near 1 has a small C, whose series is the root near
+// zero.)  With A >= 0 there is one root.
 __device__ __forceinline__ double kerr_start(double A, double C, float C2, double E2) {
   const float a = (float)A * C2;
-  if (!(fabsf(a) < 0.02f)) return E2 > 0 ? E2 * rsqrt(E2) : 0.0;
+  if (!(A >= 0 && a < 0.02f)) return E2 > 0 ? E2 * rsqrt(E2) : 0.0;
   const float q = fmaf(a, fmaf(a, fmaf(a, fmaf(a, fmaf(a, 1428.0f, -273.0f), 55.0f), -12.0f), 3.0f), -1.0f);
   return fma(C, (double)(a * q), C);
 }
 // (FP32 form: |E^n| to single precision)
 __device__ __forceinline__ double kerr_start(double A, double C, float C2, float E2) {
   const float a = (float)A * C2;
-  return fabsf(a) < 0.02f ? kerr_start(A, C, C2, 0.0) : (double)sqrtf(E2);
+  return A >= 0 && a < 0.02f ? kerr_start(A, C, C2, 0.0) : (double)sqrtf(E2);
 }
 
 // Newton solve of |E| + A |E|^3 = C, FDTD_PLRCNonlinCore::plrcStepD
