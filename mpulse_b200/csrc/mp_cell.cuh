@@ -347,8 +347,7 @@ __device__ __forceinline__ void plasma_coef(const EParams<T> &p, T sig, CellCoef
   lc.numer = lc.numer - sig;
   lc.inv_denom = T(1) / (p.denom_t + sig);
   lc.inv_denom_lo = T(0);
-  const double d = p.denom_d + (double)sig;
-  lc.chi_over_denom = p.chi_raw * (sizeof(T) == 4 ? rcp_pos1(d) : rcp_pos(d));
+  lc.chi_over_denom = p.chi_raw / (p.denom_d + (double)sig);
 }
 
 // The E update of one cell from its old E, the curl of B and the current sum:
