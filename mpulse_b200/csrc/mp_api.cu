@@ -432,7 +432,7 @@ void build_params(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, const std::vector<s
   ep.chi_d = g.chi;
   ep.chi_over_eps = g.chi / g.eps;
   ep.inv_eps = 1.0 / g.eps;
-  ep.inv_eps2 = float(ep.inv_eps * ep.inv_eps);
+  ep.inv_eps2 = ep.inv_eps * ep.inv_eps;
   ep.newton_tol = g.newton_tol;
   ep.newton_max = g.newton_max_iter;
   for (int f = 0; f < 6; ++f) {

@@ -97,26 +97,30 @@ __device__ __forceinline__ double rcp_pos1(double d) {
 
 // The start of the solves of E + A E^3 = C below.  For a = A C^2 small the reversed
 // power series E = C (1 - a + 3 a^2 - 12 a^3 + 55 a^4 - 273 a^5 + 1428 a^6 - ..)
-// (Lagrange inversion), its correction in single precision, so that E is good to
-// C (a 6e-8 + 7752 a^7) and the first Newton iteration confirms it where a is below
-// about 0.01.  Else |E^n| (E2: its square), from which a field that turns by 0.14
-// radians a step takes three.  256 x 256 x 512 Kerr FP32, steps on end at the power
-// limit: 1008 -> 967 us a step; E half of 128 x 128 x 192 with the plasma plug-ins 111
-// -> 104 us.
+// (Lagrange inversion), good to C 7752 a^7, which the first Newton iteration confirms
+// where a is below about 0.01.  Else |E^n| (E2: its square), from which a field that
+// turns by 0.14 radians a step takes three.  256 x 256 x 512 Kerr FP32, steps on end at
+// the power limit: 1008 -> 967 us a step; E half of 128 x 128 x 192 with the plasma
+// plug-ins 111 -> 104 us.
 // A < 0 always starts from |E^n|, as MPulse does (fdtd_plrc.cpp:406, fdtd_nl.cpp:86):
 // then E + A E^3 = C has three real roots, and the start decides which one is found.
 // (A static field with |A| E^2 near 1 has a small C, whose series is the root near
 // zero.)  With A >= 0 there is one root.
-__device__ __forceinline__ double kerr_start(double A, double C, float C2, double E2) {
-  const float a = (float)A * C2;
-  if (!(A >= 0 && a < 0.02f)) return E2 > 0 ? E2 * rsqrt(E2) : 0.0;
-  const float q = fmaf(a, fmaf(a, fmaf(a, fmaf(a, fmaf(a, 1428.0f, -273.0f), 55.0f), -12.0f), 3.0f), -1.0f);
+template <typename R>
+__device__ __forceinline__ double kerr_series(double C, R a) {
+  const R q = fma(a, fma(a, fma(a, fma(a, fma(a, R(1428), R(-273)), R(55)), R(-12)), R(3)), R(-1));
   return fma(C, (double)(a * q), C);
 }
-// (FP32 form: |E^n| to single precision)
+__device__ __forceinline__ double sqrt_start(double E2) { return E2 > 0 ? E2 * rsqrt(E2) : 0.0; }
+__device__ __forceinline__ double kerr_start(double A, double C, double C2, double E2) {
+  const double a = A * C2;
+  return A >= 0 && a < 0.02 ? kerr_series(C, a) : sqrt_start(E2);
+}
+// (the FP32 form of the PLRC solve: both starts in single precision, a 3e-7 added to the
+// series' error)
 __device__ __forceinline__ double kerr_start(double A, double C, float C2, float E2) {
   const float a = (float)A * C2;
-  return A >= 0 && a < 0.02f ? kerr_start(A, C, C2, 0.0) : (double)sqrtf(E2);
+  return A >= 0 && a < 0.02f ? kerr_series(C, a) : (double)sqrtf(E2);
 }
 
 // Newton solve of |E| + A |E|^3 = C, FDTD_PLRCNonlinCore::plrcStepD
@@ -377,7 +381,7 @@ __device__ __forceinline__ void e_update(const EParams<T> &p, const CellCoef<T, 
       const double rD = rsqrt(D2);  // as in the PLRC Kerr update below
       const double D = D2 * rD;
       // eps E + chi E^3 = D: E + (chi / eps) E^3 = D / eps
-      const double E0 = kerr_start(p.chi_over_eps, D * p.inv_eps, (float)D2 * p.inv_eps2, E2);
+      const double E0 = kerr_start(p.chi_over_eps, D * p.inv_eps, D2 * p.inv_eps2, E2);
       const double E = nl_newton(E0, p.eps_d, p.chi_d, D, p.newton_tol, p.newton_max, p.status, &kc.iters);
       ++kc.solves;
       const double sc = E * rD;
@@ -475,7 +479,7 @@ __device__ __forceinline__ void e_update(const EParams<T> &p, const CellCoef<T, 
         } else {
           rC = rsqrt(C2);
           C = C2 * rC;
-          E0 = kerr_start(lc.chi_over_denom, C, (float)C2, E2);
+          E0 = sizeof(T) == 4 ? sqrt_start(E2) : kerr_start(lc.chi_over_denom, C, C2, E2);
         }
         const double E = kerr_newton<sizeof(T) == 4>(E0, lc.chi_over_denom, C, p.newton_tol, p.newton_max, p.status,
                                                       &kc.iters);

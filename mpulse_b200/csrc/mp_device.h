@@ -111,8 +111,7 @@ struct EParams {
   T eps_bg, inv_eps_bg;   // background
   double chi_over_denom;  // Kerr A (PLRC nonlinear)
   double eps_d, chi_d;    // fdtd_nl
-  double chi_over_eps, inv_eps;  // chi / eps, 1 / eps and its square
-  float inv_eps2;
+  double chi_over_eps, inv_eps, inv_eps2;  // chi / eps, 1 / eps and its square
   T chi;                  // Kerr chi in the constitutive term
   double newton_tol;
   int newton_max;
