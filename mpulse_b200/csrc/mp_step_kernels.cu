@@ -597,12 +597,15 @@ constexpr int max_planes() {
 template <typename T, int V, int MODE, bool DESIGN, bool PLASMA, bool EARLY>
 static cudaError_t launch_e_np(const EParams<T> &p, int np, const HalfGrid &g, dim3 d, cudaStream_t st) {
   constexpr bool PLRC = MODE == MODE_PLRC_LIN || MODE == MODE_PLRC_NONLIN;
+  // the most poles launch_e sends here
+  constexpr int most = !PLRC ? 0 : V == 1 ? 3 : MODE == MODE_PLRC_NONLIN ? 2 : EARLY ? 1 : 3;
   const dim3 b(kRowThreads, 1, 1);
-  switch (PLRC ? np : 0) {
+  if (np > most) return cudaErrorInvalidValue;
+  switch (np) {
     case 0: return launch_pdl(e_half_kernel<T, V, MODE, 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
-    case 1: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 1 : 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
-    case 2: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 2 : 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
-    default: return launch_pdl(e_half_kernel<T, V, MODE, PLRC ? 3 : 0, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+    case 1: return launch_pdl(e_half_kernel<T, V, MODE, std::min(1, most), DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+    case 2: return launch_pdl(e_half_kernel<T, V, MODE, std::min(2, most), DESIGN, PLASMA, EARLY>, d, b, st, p, g);
+    default: return launch_pdl(e_half_kernel<T, V, MODE, most, DESIGN, PLASMA, EARLY>, d, b, st, p, g);
   }
 }
 
@@ -622,19 +625,33 @@ static cudaError_t launch_e_v(const EParams<T> &p, int np, cudaStream_t st) {
 // layers (160 x 144 x 250 124 us with one cell, 141 with two); one with the plasma
 // plug-ins (128 x 128 x 192 109 instead of 116), with a design region (96^3 21.6
 // instead of 23.0) and in FP64, whose two-cell form spills (192 x 192 x 384 551
-// instead of 691 us).  With Kerr one cell is faster by itself (128 x 128 x 256 102
-// instead of 114 us, 256 x 256 x 512 666 instead of 677), but two cells issue a
-// fifth fewer instructions: states above 1 GB, which keep the GPU at its power
-// limit, take two (256 x 256 x 512, 400 steps on end: 1032 us a step with one,
-// 1007 with two), and without the early face loads, for which it lacks registers
-// (827 us).
+// instead of 691 us).
+// Kerr: two cells issue a fifth fewer instructions, which counts where the GPU
+// works at its power limit, but lack the registers for the early face loads (827 us
+// with them on 256 x 256 x 512) and, with three poles, for the update itself (52
+// bytes spilled).  So states above 1 GB take two unless they have three poles, or x /
+// y layers in rows of less than 192 cells.  Us a step, one cell -> two, 64 steps / a
+// second of steps on end:
+//   two poles, x / y layers  256 x 256 x 512 917 -> 919 / 945 -> 934, 384 x 384 x 320
+//     1282 -> 1272 / 1318 -> 1294, 256 x 256 x 256 481 -> 484 / 493 -> 492, 192 x 192 x
+//     512 536 -> 540 / 569 -> 568, 160 x 160 x 740 546 -> 569 / 571 -> 586, 128 x 128 x
+//     1100 521 -> 527 / 527 -> 534
+//   two poles, z layers      256 x 256 x 280 477 -> 469 / 496 -> 483, 128 x 128 x 1100
+//     454 -> 446 / 461 -> 451
+//   three poles              256 x 256 x 400 927 -> 945 / 947 -> 959, 256 x 256 x 220 with
+//     z layers 478 -> 499 / 488 -> 504
+//   one pole                 256 x 256 x 400 584 -> 574 / 644 -> 622, 192 x 192 x 760 618 ->
+//     625 / 703 -> 688, 128 x 128 x 1700 631 -> 659 / 649 -> 670
+//   none                     256 x 256 x 640 711 -> 657 / 795 -> 740
+// Below, one cell: 128 x 128 x 256 with two poles 147 -> 156 / 137 -> 144, 192 x 192 x
+// 256 284 -> 281 / 289 -> 289, 256 x 256 x 128 260 -> 255 / 262 -> 257.
 template <typename T, int MODE, bool DESIGN, bool PLASMA>
 static cudaError_t launch_e(const EParams<T> &p, int np, cudaStream_t st) {
   constexpr int V = sizeof(T) == 4 && !DESIGN && !PLASMA ? 2 : 1;
-  const bool two = p.nx % V == 0 && p.nx > V &&
-                   (MODE == MODE_PLRC_NONLIN ? p.state_bytes > (1LL << 30) : !(np >= 2 && xy_faces(p)));
-  return two ? launch_e_v<T, V, MODE, DESIGN, PLASMA>(p, np, st)
-                                   : launch_e_v<T, 1, MODE, DESIGN, PLASMA>(p, np, st);
+  const bool kerr_two = np <= 2 && p.state_bytes > (1LL << 30) && (!xy_faces(p) || p.nx >= 192);
+  const bool two =
+      p.nx % V == 0 && p.nx > V && (MODE == MODE_PLRC_NONLIN ? kerr_two : !(np >= 2 && xy_faces(p)));
+  return two ? launch_e_v<T, V, MODE, DESIGN, PLASMA>(p, np, st) : launch_e_v<T, 1, MODE, DESIGN, PLASMA>(p, np, st);
 }
 
 template <typename T>

@@ -40,7 +40,8 @@ def test_linear_fp32_with_layers_matches_oracle(shape, poles):
     (258, 256, 390, 1, abi.MP_CPML_ALL),   # 1.06 GiB
     (256, 256, 740, 0, abi.MP_CPML_ALL),   # 1.08 GiB
     (130, 126, 1050, 2, abi.MP_CPML_Z),    # 1.05 GiB
-], ids=["2poles", "1pole", "vacuum", "zlayers"])
+    (256, 258, 200, 3, abi.MP_CPML_ALL),   # 1.09 GiB: three poles keep one cell per thread
+], ids=["2poles", "1pole", "vacuum", "zlayers", "3poles"])
 def test_kerr_fp32_above_1_gb_matches_fp64(nx, ny, nz, poles, cpml):
     """Six steps from smooth fields that reach into all layers, against the FP64 form
     (which test_gpu_rows and test_gpu_parity compare with the oracle): the FP32 bar
