@@ -102,6 +102,21 @@ def algorithmic_bytes(cfg: abi.Config, elem: int) -> dict:
     }
 
 
+# the E half the workload runs: two cells per thread, Kerr, two poles
+E_HALF_KERNEL = "e_half_kernel<float, 2, PLRC_NONLIN, 2>"
+
+
+def traffic_of(kernel: str, path: str | None = None):
+    """DRAM bytes of one launch of `kernel` as captured with ncu, or None when the
+    capture is of another kernel."""
+    path = path or os.path.join(ROOT, "profiles", "traffic_e_half.json")
+    if not os.path.exists(path):
+        return None
+    with open(path) as f:
+        t = json.load(f)
+    return t.get("bytes_per_launch") if t.get("kernel") == kernel else None
+
+
 def measured_peaks() -> dict:
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -360,12 +375,8 @@ def run_ours(args) -> dict:
     peaks = measured_peaks()
     e_ms = kt["e_half_ms"]
     achieved = alg["e_half"] / (e_ms / 1e3) / 1e9
-    traffic = None
-    tpath = os.path.join(ROOT, "profiles", "traffic_e_half.json")
-    if os.path.exists(tpath):
-        with open(tpath) as f:
-            traffic = json.load(f).get("bytes_per_launch")
-    roofline = {"bound": "hbm", "kernel": "e_half_kernel<float,PLRC_NONLIN,2>", "achieved": round(achieved, 1),
+    traffic = traffic_of(E_HALF_KERNEL)
+    roofline = {"bound": "hbm", "kernel": E_HALF_KERNEL, "achieved": round(achieved, 1),
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": round(achieved / peaks["hbm_gbs"], 4),
                 "traffic": traffic, "peak_source": peaks["source"],
                 "algorithmic_bytes_per_launch": alg["e_half"], "launch_ms": round(e_ms, 4)}
