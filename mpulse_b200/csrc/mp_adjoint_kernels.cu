@@ -138,9 +138,9 @@ struct AdjGrid : RowMap {
 // plane in a z entry.  On grids that exceed L2 bound by HBM and its latency (the
 // next plane is prefetched into L2), on smaller ones by instruction issue (96^3
 // with CPML on all faces: 60% of the issue slots).  Reverse step (adj_e + adj_b),
-// before -> after: 96^3 FP32 43.6 -> 40.0 us, 120 x 104 x 136 FP64 Kerr 207 -> 162,
-// 160 x 144 x 160 FP32 Kerr 229 -> 185, 256^3 FP32 Kerr 1100 -> 778, 192 x 192 x
-// 256 FP64 774 -> 546.
+// before -> after: 96^3 FP32 43.6 -> 39.7 us, 120 x 104 x 136 FP64 Kerr 207 -> 164,
+// 160 x 144 x 160 FP32 Kerr 229 -> 182, 256^3 FP32 Kerr 1100 -> 795, 192 x 192 x
+// 256 FP64 774 -> 548.
 template <typename T, int NP, bool NL>
 __global__ void __launch_bounds__(kRowThreads, adj_e_threads<T>() / kRowThreads)
     adj_e_kernel(const AdjParams<T> p, const AdjGrid g) {

@@ -859,14 +859,14 @@ int create_impl(const mp_config *cfg, mp_ctx **out) {
     if (c->fp32) c->epf.design = d;
     else c->epd.design = d;
   }
-  // AUTO = GLOBAL: on the 256x256x512 PLRC + Kerr workload the global-load
-  // kernels (E 0.92 ms, B 0.47 ms per launch) beat the TMA-staged ones
-  // (E 1.12 ms, B 0.61 ms), whose 12 small tile copies per plane and block
-  // serialise in the copy engine.
+  // AUTO = GLOBAL: on the 256x256x512 PLRC + Kerr workload (FP32) the global-load
+  // kernels (E 0.670 ms, B 0.250 ms per launch) beat the TMA-staged ones
+  // (E 0.829 ms, B 0.420 ms), whose 12 small tile copies per plane and block
+  // serialise in the copy engine, and the fused form (1.482 + 0.262 ms).
   c->fused = g.staging == MP_STAGING_FUSED;
   // CUDA graphs for grids of up to 4 M cells, where the gaps between launches
-  // matter (50 steps of 64^3 FP32 346 instead of 399 us, one step of 32^3 FP64 12
-  // instead of 19, 20 steps of 150 x 131 x 210 FP32 960 instead of 1000)
+  // matter (50 steps of 64^3 FP32 300 instead of 330 us, one step of 32^3 FP64 11.4
+  // instead of 14.7, 20 steps of 150 x 131 x 210 FP32 909 instead of 927)
   c->use_graphs = (long long)g.nx * g.ny * g.nz <= (4LL << 20);
   if (g.staging == MP_STAGING_TMA) {
     if (!setup_tma(c)) return fail(set_err(c, MP_ERR_UNSUPPORTED, "TMA tensor maps could not be encoded"));
@@ -1158,9 +1158,10 @@ int step_impl(mp_ctx *c, EParams<T> &ep, BParams<T> &bp, int n_steps, StepTimer 
       }
       // A batch that is not captured yet is launched one by one: of a long call
       // only the first 64 steps, so that the next 64 are captured and the rest
-      // replayed.  A capture costs 0.43 ms and a replayed step 0.6 to 1.4 us less
-      // (8^3 FP32 4.4 -> 3.0 us, 32^3 FP64 5.1 -> 4.4, 64^3 FP32 6.8 -> 6.0, 128^3
-      // 24.5 -> 23.8), so it takes some 600 steps to earn.
+      // replayed.  A capture costs 0.43 ms and a replayed step 0.4 to 1.4 us less, so
+      // it takes some 600 steps to earn.  A first call of 1000 steps, all one by one ->
+      // so, us a step: 8^3 FP32 7.4 -> 3.7, 16^3 5.0 -> 4.3, 32^3 FP64 5.1 -> 5.15, 64^3
+      // FP32 6.6 -> 6.3, 128^3 24.3 -> 23.8; of 4000 steps of 64^3 6.6 -> 6.0.
       if (!c->nsrc && K > Kg + 640) K = Kg;
     }
     for (int q = 0; q < K; ++q) {

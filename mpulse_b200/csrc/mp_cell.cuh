@@ -1,10 +1,12 @@
-// mp_cell.cuh - the arithmetic of one cell's E update and B update, shared by
-// the global-load kernels (mp_step_kernels.cu) and the TMA-staged kernels
-// (mp_step_tma.cu).  The caller loads the field values (from global memory or
-// from shared memory) and the PLRC accumulators, calls e_cell / b_cell, and
-// stores the results; the CPML psi of the faces containing the cell and the
-// injection-plane values are loaded and stored here with plain global accesses
-// (a minority of cells).
+// mp_cell.cuh - the arithmetic of one cell's E update and B update.  All kernel
+// forms share the coefficients (cell_coef, plasma_coef), the E update (e_update)
+// and the sums of products; the half-step kernels (mp_step_kernels.cu) load and
+// add the CPML faces of a thread's cells themselves.  In the TMA-staged and fused
+// kernels (mp_step_tma.cu, mp_step_fused.cu) the caller loads the field values
+// (from global or shared memory) and the PLRC accumulators, calls e_cell / b_cell,
+// and stores the results; the CPML psi of the faces containing the cell and the
+// injection-plane values are then loaded and stored here with plain global
+// accesses (a minority of cells).
 //
 // Order of operations per cell: every load before any store.  The arrays may
 // alias as far as the compiler can tell, so a load written after a store would

@@ -26,17 +26,17 @@
 // grids that exceed L2 both kernels are bound by HBM, on smaller ones by the
 // instructions they issue (before this form 541 per 32 cells in the E half and
 // 394 in the B half of a 96^3 grid with CPML on all faces, issue slots 68% and
-// 60% busy; now 387 and 257), which is why the faces are found from six
+// 60% busy; now 390 and 170), which is why the faces are found from six
 // thresholds, rows from a multiplication, and nothing is tested per cell that is
 // fixed per thread or per plane.  On large grids the loads of one plane per
 // warp do not cover the latency of HBM: the next plane's lines are prefetched
 // into L2 while this plane is computed, which needs no registers.
 // Measured per half step, before -> after (B200, us):
-//   256 x 256 x 512 PLRC + Kerr FP32   E 758 -> 666   B 276 -> 250
-//   192 x 192 x 384 PLRC + Kerr FP64   E 659 -> 547   B 225 -> 199
-//   150 x 131 x 210 fdtd-plain FP32    E  37 ->  28   B  48 ->  29
-//   101 x 75 x 163 fdtd-nl FP64        E  49 ->  24   B  40 ->  16
-//   128 x 128 x 192 + plasma FP32      E 135 -> 106   B  56 ->  37
+//   256 x 256 x 512 PLRC + Kerr FP32   E 758 -> 670   B 276 -> 250
+//   192 x 192 x 384 PLRC + Kerr FP64   E 659 -> 549   B 225 -> 197
+//   150 x 131 x 210 fdtd-plain FP32    E  37 ->  30   B  48 ->  31
+//   101 x 75 x 163 fdtd-nl FP64        E  49 ->  23   B  40 ->  17
+//   128 x 128 x 192 + plasma FP32      E 135 ->  98   B  56 ->  37
 #include "mp_cell.cuh"
 #include "mp_pdl.cuh"
 #include "mp_row.cuh"
@@ -47,7 +47,8 @@ namespace mpb {
 
 // Resident threads per SM asked of the register allocator.  E half: FP32 with
 // one cell per thread 1024 (64 registers; 896: 687 instead of 666 us on 256 x 256 x
-// 512), with the plasma plug-ins 896 (106 instead of 114 us on 128 x 128 x 192),
+// 512 run with one cell), with the plasma plug-ins 896 (106 instead of 114 us on 128 x
+// 128 x 192),
 // with two cells 768 (80 registers); FP64 640 (96 registers; 768 spill: 96
 // instead of 87 us with a design region, 120 x 104 x 136).  B half: FP32 1280 (48
 // registers; 1024: 264 instead of 257 us on 256 x 256 x 512), with the faces
@@ -150,8 +151,8 @@ __device__ __forceinline__ void face_currents(const CpmlFace<T> (&cpml)[6], int 
 // in the same order.  face_currents waits once per face, and a warp with x-face
 // cells does so on every plane.  B half with CPML on all faces (FP32, us): 96^3
 // 18.8 -> 14.1, 128 x 128 x 192 44 -> 37, 128 x 128 x 256 54 -> 45, 256 x 256 x 512
-// 260 -> 250; E half 128 x 128 x 256 Kerr 107 -> 102, 256 x 256 x 512 676 -> 666,
-// 101 x 131 x 120 with two poles 49 -> 43, FP64 120 x 104 x 136 87 -> 82.  Grids
+// 260 -> 250; E half 128 x 128 x 256 Kerr 107 -> 102, 101 x 131 x 120 with two poles
+// 49 -> 43, FP64 120 x 104 x 136 87 -> 82.  Grids
 // without x / y layers keep face_currents, which needs fewer registers (160 x 144
 // x 250 with z layers, B half 44 us; with the early loads 50), and so do grids
 // whose layers meet.
@@ -559,13 +560,13 @@ static bool xy_faces(const P &p) {
 
 // The grid of a half step: V cells per thread, z-chunks of the planes.
 // Planes per block: one where two would leave SMs without four blocks (32^3
-// FP64: E 9.1 instead of 10.2 us; 72^3 12.2 instead of 13.1 us a step); else at least two, and more while 50 blocks
-// per SM remain, up to max_planes.  Longer chunks save the two carried loads of
+// FP64: E 9.1 instead of 10.2 us; 72^3 12.2 instead of 13.1 us a step); else at least
+// two, and more while 50 blocks per SM remain, up to max_planes.  Longer chunks save the two carried loads of
 // each chunk's first plane but leave fewer warps and a longer tail (256 x 256 x
-// 512 FP32 E half with 2 / 4 / 8 / 16 / 24 planes 725 / 682 / 677 / 700 / 715 us,
-// 128 x 128 x 256 112 / 107 / 112 us with 2 / 4 / 8).  The prefetch is for
-// states that do not stay in L2 (126 MB): 256 x 256 x 512 E half 748 -> 677 us,
-// 120 x 104 x 136 FP64 93 -> 89; on a 99 MB state 29.8 -> 31.5.
+// 512 FP32 E half, one cell per thread, with 2 / 4 / 8 / 16 / 24 planes 725 / 682 /
+// 677 / 700 / 715 us, 128 x 128 x 256 112 / 107 / 112 us with 2 / 4 / 8).  The prefetch
+// is for states that do not stay in L2 (126 MB): 256 x 256 x 512 E half, one cell, 748
+// -> 677 us, 120 x 104 x 136 FP64 93 -> 89; on a 99 MB state 29.8 -> 31.5.
 template <typename P>
 static HalfGrid row_grid(const P &p, int V, int max_planes, dim3 *d) {
   HalfGrid r;
@@ -626,8 +627,8 @@ static cudaError_t launch_e_v(const EParams<T> &p, int np, cudaStream_t st) {
 // plug-ins (128 x 128 x 192 109 instead of 116), with a design region (96^3 21.6
 // instead of 23.0) and in FP64, whose two-cell form spills (192 x 192 x 384 551
 // instead of 691 us).
-// Kerr: two cells issue a fifth fewer instructions, which counts where the GPU
-// works at its power limit, but lack the registers for the early face loads (827 us
+// Kerr: two cells issue 27% fewer instructions (256 x 256 x 320 223 instead of 307 M),
+// which counts where the GPU works at its power limit, but lack the registers for the early face loads (827 us
 // with them on 256 x 256 x 512) and, with three poles, for the update itself (52
 // bytes spilled).  So states above 1 GB take two unless they have three poles, or x /
 // y layers in rows of less than 192 cells.  Us a step, one cell -> two, 64 steps / a
